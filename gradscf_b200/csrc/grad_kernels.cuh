@@ -349,9 +349,13 @@ __global__ void __launch_bounds__(128, 3) grad_reg_kernel(JKArgs args) {
   int atA = 0, atB = 0;
   int kb, ke;
   grad_ket_range(args, item, w, kb, ke);
-  for (int k0 = kb; k0 < ke; k0 += 32) {
-    const bool active = k0 + lane < ke;
-    const int k = active ? k0 + lane : ke - 1;
+  if (kb >= ke) return;
+  // few kets in the item: groups of lanes share each quartet's primitives
+  const LaneSplit ls = lane_split(lane, ke - kb, args.pair_info[bra].w, args.pair_info[args.ket_pairs[kb]].w);
+  const int slot = lane / ls.t;
+  for (int k0 = kb; k0 < ke; k0 += 32 / ls.t) {
+    const bool active = k0 + slot < ke;
+    const int k = active ? k0 + slot : ke - 1;
     QuartetGeom g;
     load_quartet(args, bra, args.ket_pairs[k], g);
     atA = args.ws_atm[g.A];
@@ -366,9 +370,9 @@ __global__ void __launch_bounds__(128, 3) grad_reg_kernel(JKArgs args) {
       gam[o] = active ? R(g.scale * gamma_abcd(args, base, n, g.aoA + ia, g.aoB + ib, g.aoC + ic, g.aoD + id)) : R(0);
     });
     R dA[3] = {0, 0, 0}, dB[3] = {0, 0, 0}, dC[3] = {0, 0, 0};
-    for (int i = g.ppa; i < g.ppa + g.npa; ++i) {
+    for (int i = g.ppa + ls.si; i < g.ppa + g.npa; i += ls.ti) {
       const R alpha = R(args.pp_exp[i].x), beta = R(args.pp_exp[i].y);
-      for (int j = g.ppc; j < g.ppc + g.npc; ++j) {
+      for (int j = g.ppc + ls.sj; j < g.ppc + g.npc; j += ls.tj) {
         PrimQ<R> s;
         grad_prim<R>(args, g, i, j, s);
         const R gamma_c = R(args.pp_exp[j].x);
@@ -413,7 +417,10 @@ __global__ void __launch_bounds__(128, 3) grad_reg_kernel(JKArgs args) {
         }
       }
     }
-    if (active) {
+    lane_sum<3>(dA, ls);
+    lane_sum<3>(dB, ls);
+    lane_sum<3>(dC, ls);
+    if (active && ls.sub == 0) {
       double* gC = args.grad + 3LL * args.ws_atm[g.C];
       double* gD = args.grad + 3LL * args.ws_atm[g.D];
 #pragma unroll
@@ -726,9 +733,13 @@ __global__ void __launch_bounds__(128) grad_lane_kernel(JKArgs args) {
   int atA = 0, atB = 0;
   int kb, ke;
   grad_ket_range(args, item, w, kb, ke);
-  for (int k0 = kb; k0 < ke; k0 += 32) {
-    const bool active = k0 + lane < ke;
-    const int k = active ? k0 + lane : ke - 1;
+  if (kb >= ke) return;
+  // few kets in the item: groups of lanes share each quartet's primitives
+  const LaneSplit ls = lane_split(lane, ke - kb, args.pair_info[bra].w, args.pair_info[args.ket_pairs[kb]].w);
+  const int slot = lane / ls.t;
+  for (int k0 = kb; k0 < ke; k0 += 32 / ls.t) {
+    const bool active = k0 + slot < ke;
+    const int k = active ? k0 + slot : ke - 1;
     QuartetGeom g;
     load_quartet(args, bra, args.ket_pairs[k], g);
     atA = args.ws_atm[g.A];
@@ -742,9 +753,9 @@ __global__ void __launch_bounds__(128) grad_lane_kernel(JKArgs args) {
           active ? R(g.scale * gamma_abcd(args, base, n, g.aoA + ia, g.aoB + ib, g.aoC + ic, g.aoD + id)) : R(0);
     }
     R dA[3] = {0, 0, 0}, dB[3] = {0, 0, 0}, dC[3] = {0, 0, 0};
-    for (int i = g.ppa; i < g.ppa + g.npa; ++i) {
+    for (int i = g.ppa + ls.si; i < g.ppa + g.npa; i += ls.ti) {
       const R alpha = R(args.pp_exp[i].x), beta = R(args.pp_exp[i].y);
-      for (int j = g.ppc; j < g.ppc + g.npc; ++j) {
+      for (int j = g.ppc + ls.sj; j < g.ppc + g.npc; j += ls.tj) {
         PrimQ<R> s;
         grad_prim<R>(args, g, i, j, s);
         const R gamma_c = R(args.pp_exp[j].x);
@@ -764,7 +775,10 @@ __global__ void __launch_bounds__(128) grad_lane_kernel(JKArgs args) {
         }
       }
     }
-    if (active) {
+    lane_sum<3>(dA, ls);
+    lane_sum<3>(dB, ls);
+    lane_sum<3>(dC, ls);
+    if (active && ls.sub == 0) {
       double* gC = args.grad + 3LL * args.ws_atm[g.C];
       double* gD = args.grad + 3LL * args.ws_atm[g.D];
 #pragma unroll

@@ -738,6 +738,25 @@ static int reg_chunk(long long npa, long long npc) {
   return npa * npc >= (long long)(B200JK_HEAVY_PQ) ? 32 : B200JK_REG_CHUNK;
 }
 
+// Items of a launch with too little work to fill the device are cut smaller:
+// an item holds at most 1/kItemsPerLaunch of the launch's primitive quartets
+// (about three per resident warp of the register kernels, 148 x 20 warps),
+// but at least kItemFloor of them, where its fixed latency (queue, records,
+// adds) starts to show.  Launches of more than kItemsPerLaunch full items keep
+// the full shape.  Measured with the lane sharing of jk_kernels.cuh: water
+// cc-pVDZ FP64 build 3.02 -> 0.81 ms, (H2O)8 7.92 -> 4.05 ms, (H2O)4 cc-pVTZ
+// force 68.8 -> 49.2 ms, (H2O)32 split build (full items) 57.7 -> 53.9 ms.
+constexpr long long kItemsPerLaunch = 9472, kItemFloor = 256;
+static long long item_budget(long long total) { return std::max(kItemFloor, total / kItemsPerLaunch); }
+
+// Kets per register-path item of `wq` primitive quartets each: below 32 only
+// as far as groups of lanes (lane_split) keep four primitive quartets a lane.
+static int shrink_kets(int nk, long long wq, long long budget) {
+  while (nk > 32 && nk * wq > budget) nk /= 2;
+  while (nk > 1 && nk <= 32 && nk * wq > budget && wq * nk >= 256) nk /= 2;
+  return nk;
+}
+
 static void upload_items(DevBuf& work, DevBuf& split, const std::vector<int4>& items) {
   CUDA_OK(work.ensure(std::max<size_t>(items.size(), 1) * sizeof(int4)));
   if (!items.empty())
@@ -768,8 +787,10 @@ static int screen_end(const ClassList& Y, int lo, int hi, double qb, double cut)
 // same molecule (entries with `gk` combinations), the kets any bra of the
 // group meets (its Schwarz prefix, and at most its own position when X and
 // Y are one list), cut into chunks.
-static void fill_group(GroupWork& G, const ClassList& X, const ClassList& Y, bool same, double cut, int chunk,
-                       int gb, int gk) {
+// `total`: the launch's primitive quartets (item_budget).
+static void fill_group(GroupWork& G, const ClassList& X, const ClassList& Y, bool same, double cut, int chunk0,
+                       int gb, int gk, long long total) {
+  const long long budget = item_budget(total);
   G.all_items.clear();
   G.h_items.clear();
   G.item_cost.clear();
@@ -781,11 +802,17 @@ static void fill_group(GroupWork& G, const ClassList& X, const ClassList& Y, boo
     const int first = X.bord[g0];
     if (nco(X, first) != gb) continue;
     const int m = X.mol_pos[first];
-    for (int c0 = g0; c0 < g1; c0 += B200JK_GRP_BRAS) {
-      const int c1 = std::min(g1, c0 + B200JK_GRP_BRAS);
-      for (const int2 seg : Y.segs[m]) {
-        const int lo = seg.x;
-        if (nco(Y, lo) != gk) continue;
+    for (const int2 seg : Y.segs[m]) {
+      const int lo = seg.x;
+      if (nco(Y, lo) != gk) continue;
+      // the item's shape: full passes first, then fewer bras, then fewer kets
+      const long long wq = (long long)X.npp_pos[first] * Y.npp_pos[lo];
+      int chunk = chunk0, bras = B200JK_GRP_BRAS;
+      while (chunk > 32 && bras * chunk * wq > budget) chunk /= 2;
+      while (bras > 1 && bras * chunk * wq > budget) bras /= 2;
+      chunk = shrink_kets(chunk, wq, budget);
+      for (int c0 = g0; c0 < g1; c0 += bras) {
+        const int c1 = std::min(g1, c0 + bras);
         hp.assign(c1 - c0, lo);
         int hi = lo;
         for (int i = c0; i < c1; ++i) {
@@ -877,19 +904,32 @@ static void fill_items(Plan& p, ClassPairWork& W, int force) {
   std::vector<int4> items;
   W.quartets = W.prim_quartets = 0;
   W.item_cost.clear();
+  std::vector<int4> runs;   // (bra position, ket begin, ket end), reused by the item loop
   for_each_run(X, Y, x == y, cut, [&](int bp, int lo, int hi) {
-    const long long npa = X.npp_pos[bp];
-    int chunk = chunk0;
-    if (disp.tile[cls] && B200JK_TILE_CHUNK > 0) chunk = B200JK_TILE_CHUNK;
-    else if (disp.reg_path[cls]) chunk = (force > 0 && !grouped) ? force : reg_chunk(npa, Y.npp_pos[lo]);
     W.quartets += hi - lo;
-    W.prim_quartets += npa * (Y.npp_prefix[hi] - Y.npp_prefix[lo]);
+    W.prim_quartets += (long long)X.npp_pos[bp] * (Y.npp_prefix[hi] - Y.npp_prefix[lo]);
+    runs.push_back(make_int4(bp, lo, hi, 0));
+  });
+  const long long budget = item_budget(W.prim_quartets);
+  // one block per item: about four per resident block (148 x 8)
+  const long long block_budget = W.prim_quartets / 4736;
+  for (const int4& r : runs) {
+    const int bp = r.x, lo = r.y, hi = r.z;
+    const long long npa = X.npp_pos[bp], wq = npa * Y.npp_pos[lo];
+    int chunk = chunk0;
+    if (disp.reg_path[cls]) {
+      chunk = shrink_kets((force > 0 && !grouped) ? force : reg_chunk(npa, Y.npp_pos[lo]), wq, budget);
+    } else {
+      // blocks of several quartets (tile, team) or of one (grad_block_kernel)
+      if (disp.tile[cls] && B200JK_TILE_CHUNK > 0) chunk = B200JK_TILE_CHUNK;
+      while (chunk > 1 && chunk * wq > block_budget) chunk /= 2;
+    }
     for (int s = lo; s < hi; s += chunk) {
       const int e = std::min(hi, s + chunk);
       items.push_back(make_int4(bp, s, e, 0));
       W.item_cost.push_back(npa * (Y.npp_prefix[e] - Y.npp_prefix[s]));
     }
-  });
+  }
   W.nwork = (int)items.size();
   ++p.layout_gen;
   upload_items(W.work, W.split, items);
@@ -900,11 +940,12 @@ static void fill_items(Plan& p, ClassPairWork& W, int force) {
   const bool grp = disp.grp64[cls] && disp.grp32[cls];
   const int gchunk0 = force > 0 ? force : B200JK_GRP_CHUNK;
   W.use_grp = grp && !grouped;
-  if (W.use_grp) fill_group(W.grp, X, Y, x == y, cut, gchunk0, 1, 1);
+  if (W.use_grp) fill_group(W.grp, X, Y, x == y, cut, gchunk0, 1, 1, W.prim_quartets);
   if (!grouped) return;
   const ClassList& GX = W.grouped_x ? p.grouped[x] : X;
   const ClassList& GY = W.grouped_y ? p.grouped[y] : Y;
   std::map<std::pair<int, int>, GenBucket*> by;
+  runs.clear();
   for_each_run(GX, GY, x == y, cut, [&](int bp, int lo, int hi) {
     const int gb = GX.nco.empty() ? 1 : GX.nco[bp];
     const int gk = GY.nco.empty() ? 1 : GY.nco[lo];
@@ -914,16 +955,22 @@ static void fill_items(Plan& p, ClassPairWork& W, int force) {
       B->gb = gb;
       B->gk = gk;
     }
-    const long long npa = GX.npp_pos[bp];
     B->quartets += (long long)(hi - lo) * gb * gk;
-    B->prim_quartets += npa * (GY.npp_prefix[hi] - GY.npp_prefix[lo]);
-    const int gchunk = force > 0 ? force : reg_chunk(npa, GY.npp_pos[lo]);
+    B->prim_quartets += (long long)GX.npp_pos[bp] * (GY.npp_prefix[hi] - GY.npp_prefix[lo]);
+    runs.push_back(make_int4(bp, lo, hi, 0));
+  });
+  for (const int4& r : runs) {
+    const int bp = r.x, lo = r.y, hi = r.z;
+    GenBucket* B = by[{GX.nco.empty() ? 1 : GX.nco[bp], GY.nco.empty() ? 1 : GY.nco[lo]}];
+    const long long npa = GX.npp_pos[bp];
+    const int gchunk = shrink_kets(force > 0 ? force : reg_chunk(npa, GY.npp_pos[lo]), npa * GY.npp_pos[lo],
+                                   item_budget(B->prim_quartets));
     for (int s = lo; s < hi; s += gchunk) {
       const int e = std::min(hi, s + gchunk);
       B->all_items.push_back(make_int4(bp, s, e, 0));
-      B->item_cost.push_back(npa * (GY.npp_prefix[e] - GY.npp_prefix[s]) * (gb * gk > 1 ? 2 : 1));
+      B->item_cost.push_back(npa * (GY.npp_prefix[e] - GY.npp_prefix[s]) * (B->gb * B->gk > 1 ? 2 : 1));
     }
-  });
+  }
   for (auto& kv : by) {
     GenBucket* B = kv.second;
     B->h_items.clear();
@@ -934,7 +981,7 @@ static void fill_items(Plan& p, ClassPairWork& W, int force) {
                                                        disp.grpg32[cls][gen_slot(B->gb, B->gk)] != nullptr);
     if (bgrp) {
       B->use_grp = true;
-      fill_group(B->grp, GX, GY, x == y, cut, gchunk0, B->gb, B->gk);
+      fill_group(B->grp, GX, GY, x == y, cut, gchunk0, B->gb, B->gk, B->prim_quartets);
     }
     W.buckets.push_back(B);
   }

@@ -320,7 +320,53 @@ __device__ __forceinline__ long long dm_index(const JKArgs& args, int mol, int a
 }
 
 // ---------------------------------------------------------------------------
-// Register path: one thread per quartet, the whole Cartesian block in registers.
+// Lane sharing.  A work item's kets have one primitive-pair count, so when an
+// item holds fewer kets than a warp has lanes, T = 32 / (kets, rounded up to
+// a power of two) neighbouring lanes share each quartet: lane `sub` of the T
+// takes the bra primitives sub % ti, + ti, ... and the ket primitives
+// sub / ti, + tj, ... (ti tj = T), and the partial blocks are added by
+// shuffles before digestion, which the group's first lane does.  What bounds
+// a small build is the longest chain of dependent primitive quartets, not
+// throughput: water cc-pVDZ spent 1.5 of its 3.1 ms in one lane walking the
+// 4096 primitive quartets of the oxygen core (ss|ss) block.  T is kept where
+// every lane of the group gets at least two primitive quartets.
+// ---------------------------------------------------------------------------
+struct LaneSplit {
+  int t = 1, sub = 0;              // lanes per quartet, this lane's index among them
+  int ti = 1, si = 0, tj = 1, sj = 0;
+  unsigned mask = 0;               // the group's lanes
+};
+
+__device__ __forceinline__ LaneSplit lane_split_t(int lane, int t, int npa) {
+  LaneSplit s;
+  s.t = t;
+  s.sub = lane & (t - 1);
+  s.ti = min(t, 1 << (31 - __clz(max(npa, 1))));
+  s.tj = t / s.ti;
+  s.si = s.sub & (s.ti - 1);
+  s.sj = s.sub / s.ti;
+  s.mask = t == 32 ? 0xffffffffu : ((1u << t) - 1u) << (lane & ~(t - 1));
+  return s;
+}
+
+__device__ __forceinline__ LaneSplit lane_split(int lane, int nkets, int npa, int npc) {
+  int t = 1;
+  while (t < 32 && nkets * t <= 16 && npa * npc >= 4 * t) t *= 2;
+  return lane_split_t(lane, t, npa);
+}
+
+// Sum of v[0..N) over the lanes of the group, in every one of them.
+template <int N, typename R>
+__device__ __forceinline__ void lane_sum(R* v, const LaneSplit& s) {
+  for (int off = 1; off < s.t; off <<= 1) {
+#pragma unroll
+    for (int o = 0; o < N; ++o) v[o] += __shfl_xor_sync(s.mask, v[o], off);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Register path: one thread (or one group of lanes, above) per quartet, the
+// whole Cartesian block in registers.
 // ---------------------------------------------------------------------------
 #ifndef B200JK_REG_UNROLL
 #define B200JK_REG_UNROLL 2
@@ -330,7 +376,7 @@ template <int LA, int LB, int LC, int LD, typename R>
 __device__ __forceinline__ void quartet_block_reg(const JKArgs& args, const QuartetGeom& g,
                                                   const typename PrimData<R>::A* bpp,
                                                   const typename PrimData<R>::B* baux, R* out,
-                                                  const float* s_boys) {
+                                                  const float* s_boys, const LaneSplit& ls) {
   using CI = ClassInfo<LA, LB, LC, LD>;
   using GI = GIdx<LA, LB, LC, LD>;
   constexpr int N = CI::NROOT;
@@ -340,17 +386,19 @@ __device__ __forceinline__ void quartet_block_reg(const JKArgs& args, const Quar
   // shared memory (inner): one global read per ket primitive pair.
   const float3 ac = make_float3(float(g.ax - g.cx), float(g.ay - g.cy), float(g.az - g.cz));
   // the next ket primitive is fetched while the current one is in use
-  auto Qn = PrimData<R>::a(args, g.ppc);
-  auto QAn = PrimData<R>::b(args, g.ppc);
-  for (int j = g.ppc; j < g.ppc + g.npc; ++j) {
+  const int jl = g.ppc + g.npc;
+  int j = min(g.ppc + ls.sj, jl - 1);
+  auto Qn = PrimData<R>::a(args, j);
+  auto QAn = PrimData<R>::b(args, j);
+  for (j = g.ppc + ls.sj; j < jl; j += ls.tj) {
     const auto Q = Qn;
     const auto QA = QAn;
-    if (j + 1 < g.ppc + g.npc) {
-      Qn = PrimData<R>::a(args, j + 1);
-      QAn = PrimData<R>::b(args, j + 1);
+    if (j + ls.tj < jl) {
+      Qn = PrimData<R>::a(args, j + ls.tj);
+      QAn = PrimData<R>::b(args, j + ls.tj);
     }
 #pragma unroll(kRegUnroll)
-    for (int i = 0; i < g.npa; ++i) {
+    for (int i = ls.si; i < g.npa; i += ls.ti) {
       PrimQ<R> s;
       prim_any<R>(g, ac, bpp[i], baux[i], Q, QA, s);
       R x[N], w[N];
@@ -381,6 +429,7 @@ __device__ __forceinline__ void quartet_block_reg(const JKArgs& args, const Quar
       }
     }
   }
+  lane_sum<CI::NOUT>(out, ls);
 }
 
 // Density elements one quartet digests, in a fixed order: D[c][d] (J of the
@@ -613,16 +662,18 @@ __global__ void __launch_bounds__(128, (RegMinBlocks<LA, LB, LC, LD, R>::value))
   const PB_t* baux = cached ? s_aux[warp] : (sizeof(R) == 4 ? (const PB_t*)(args.pp_f2 + ppb)
                                                            : (const PB_t*)(args.pp_aux + ppb));
   QuartetGeom g;
-  for (int k0 = kb; k0 < ke; k0 += 32) {
+  const LaneSplit ls = lane_split(lane, ke - kb, npb, args.ket_ix[kb].y);
+  const int slot = lane / ls.t;
+  for (int k0 = kb; k0 < ke; k0 += 32 / ls.t) {
     // lanes past the range recompute the last ket with their output masked,
     // so the whole warp takes part in the J shuffles
-    const bool active = k0 + lane < ke;
-    const int k = active ? k0 + lane : ke - 1;
+    const bool valid = k0 + slot < ke, active = valid && ls.sub == 0;
+    const int k = valid ? k0 + slot : ke - 1;
     load_quartet_rec(args, br, k, g);
     DensPre<LA, LB, LC, LD, R> pre;
     pre.load(args, g);
     R out[CI::NOUT];
-    quartet_block_reg<LA, LB, LC, LD, R>(args, g, bpp, baux, out, s_boys);
+    quartet_block_reg<LA, LB, LC, LD, R>(args, g, bpp, baux, out, s_boys, ls);
     digest_reg<LA, LB, LC, LD, R>(args, g, out, acc_j, active, s_jab[warp], pre);
   }
   if (acc_j) {
@@ -792,9 +843,11 @@ __global__ void __launch_bounds__(128, (RegMinBlocks<LA, LB, LC, LD, R>::value))
   auto dv = [&](int r, int c) -> R { return __ldg(dm0 + (long long)r * n + c); };
   const bool doj = args.with_j != 0 && args.nsym > 0, dok = args.with_k != 0;
   R(*acc)[32] = s_acc[warp];
-  for (int k0 = w.z; k0 < w.w; k0 += 32) {
-    const bool valid = k0 + lane < w.w;
-    const int k = valid ? k0 + lane : w.w - 1;
+  const LaneSplit ls = lane_split(lane, w.w - w.z, args.bra_ix[p0].y, args.ket_ix[w.z].y);
+  const int slot = lane / ls.t;
+  for (int k0 = w.z; k0 < w.w; k0 += 32 / ls.t) {
+    const bool valid = k0 + slot < w.w;
+    const int k = valid ? k0 + slot : w.w - 1;
     const double qk = args.ket_q[k];
     const double4 kra = args.ket_ra[k], kab = args.ket_ab[k];
     const int4 kix = args.ket_ix[k];
@@ -805,7 +858,7 @@ __global__ void __launch_bounds__(128, (RegMinBlocks<LA, LB, LC, LD, R>::value))
     for (int bi = 0; bi < w.y; ++bi) {
       const int pos = bord[w.x + bi];
       const double qq = args.bra_q[pos] * qk;
-      bool act = valid && qq >= cut && (!args.same_list || k <= pos);
+      bool act = valid && ls.sub == 0 && qq >= cut && (!args.same_list || k <= pos);
       if (args.split_mode == 1) act = act && !(qq * qm < args.fp32_cut);
       else if (args.split_mode == 2) act = act && (qq * qm < args.fp32_cut);
       if (!__any_sync(0xffffffffu, act)) continue;
@@ -836,7 +889,7 @@ __global__ void __launch_bounds__(128, (RegMinBlocks<LA, LB, LC, LD, R>::value))
       g.scale = (aoA == br.ix.w ? 0.5 : 1.0) * (aoC == aoD ? 0.5 : 1.0) * (args.same_list && k == pos ? 0.5 : 1.0);
       g.omega2 = args.omega2;
       R out[CI::NOUT];
-      quartet_block_reg<LA, LB, LC, LD, R>(args, g, bpp, baux, out, s_boys);
+      quartet_block_reg<LA, LB, LC, LD, R>(args, g, bpp, baux, out, s_boys, ls);
       const int aoB = br.ix.w;
       const R sR = act ? R(g.scale) : R(0);
 #define V_(a, b, c, d) (out[(((a) * NB + (b)) * NC + (c)) * ND + (d)])
@@ -987,29 +1040,31 @@ __device__ __forceinline__ void quartet_block_gen(const JKArgs& args, const Quar
                                                   const typename PrimData<R>::A* bpp,
                                                   const typename PrimData<R>::B* baux,
                                                   const typename CoefSel<R>::T* bco, R* out,
-                                                  const float* s_boys) {
+                                                  const float* s_boys, const LaneSplit& ls) {
   using CI = ClassInfo<LA, LB, LC, LD>;
   using GI = GIdx<LA, LB, LC, LD>;
   constexpr int N = CI::NROOT, NO = CI::NOUT;
 #pragma unroll
   for (int o = 0; o < GB * GK * NO; ++o) out[o] = R(0);
   const float3 ac = make_float3(float(g.ax - g.cx), float(g.ay - g.cy), float(g.az - g.cz));
-  auto Qn = PrimData<R>::a(args, g.ppc);
-  auto QAn = PrimData<R>::b(args, g.ppc);
-  auto Cn = CoefSel<R>::get(args, g.ppc);
-  for (int j = g.ppc; j < g.ppc + g.npc; ++j) {
+  const int jl = g.ppc + g.npc;
+  int j = min(g.ppc + ls.sj, jl - 1);
+  auto Qn = PrimData<R>::a(args, j);
+  auto QAn = PrimData<R>::b(args, j);
+  auto Cn = CoefSel<R>::get(args, j);
+  for (j = g.ppc + ls.sj; j < jl; j += ls.tj) {
     const auto Q = Qn;
     const auto QA = QAn;
     const auto CK = Cn;
-    if (j + 1 < g.ppc + g.npc) {
-      Qn = PrimData<R>::a(args, j + 1);
-      QAn = PrimData<R>::b(args, j + 1);
-      Cn = CoefSel<R>::get(args, j + 1);
+    if (j + ls.tj < jl) {
+      Qn = PrimData<R>::a(args, j + ls.tj);
+      QAn = PrimData<R>::b(args, j + ls.tj);
+      Cn = CoefSel<R>::get(args, j + ls.tj);
     }
     R sb[PRESUM ? GB * NO : 1];
 #pragma unroll
     for (int o = 0; o < (PRESUM ? GB * NO : 1); ++o) sb[o] = R(0);
-    for (int i = 0; i < g.npa; ++i) {
+    for (int i = ls.si; i < g.npa; i += ls.ti) {
       PrimQ<R> s;
       prim_any<R>(g, ac, bpp[i], baux[i], Q, QA, s);
       R x[N], w[N];
@@ -1074,6 +1129,7 @@ __device__ __forceinline__ void quartet_block_gen(const JKArgs& args, const Quar
       });
     }
   }
+  lane_sum<GB * GK * NO>(out, ls);
 }
 
 template <int LA, int LB, int LC, int LD, typename R, int GB, int GK>
@@ -1141,9 +1197,11 @@ __global__ void __launch_bounds__(128, (RegMinBlocks<LA, LB, LC, LD, R,
   const C4* bco = cached ? s_co[warp] : (sizeof(R) == 4 ? (const C4*)(args.pp_cf + ppb)
                                                        : (const C4*)(args.pp_c + ppb));
   QuartetGeom g;
-  for (int k0 = kb; k0 < ke; k0 += 32) {
-    const bool active = k0 + lane < ke;
-    const int k = active ? k0 + lane : ke - 1;
+  const LaneSplit ls = lane_split(lane, ke - kb, npb, args.ket_ix[kb].y);
+  const int slot = lane / ls.t;
+  for (int k0 = kb; k0 < ke; k0 += 32 / ls.t) {
+    const bool valid = k0 + slot < ke, active = valid && ls.sub == 0;
+    const int k = valid ? k0 + slot : ke - 1;
     load_quartet_rec(args, br, k, g);
     int aoC[GK], aoD[GK];
     bool kdiag;
@@ -1160,7 +1218,7 @@ __global__ void __launch_bounds__(128, (RegMinBlocks<LA, LB, LC, LD, R,
     }
     const double sbk = (bdiag ? 0.5 : 1.0) * (kdiag ? 0.5 : 1.0) * (args.same_list && k == w.x ? 0.5 : 1.0);
     R out[GB * GK * NO];
-    quartet_block_gen<LA, LB, LC, LD, R, GB, GK>(args, g, bpp, baux, bco, out, s_boys);
+    quartet_block_gen<LA, LB, LC, LD, R, GB, GK>(args, g, bpp, baux, bco, out, s_boys, ls);
 #pragma unroll
     for (int b = 0; b < GB; ++b)
 #pragma unroll
@@ -1264,9 +1322,11 @@ __global__ void __launch_bounds__(128, (RegMinBlocks<LA, LB, LC, LD, R,
   auto dv = [&](int r, int c) -> R { return __ldg(dm0 + (long long)r * n + c); };
   const bool doj = args.with_j != 0 && args.nsym > 0, dok = args.with_k != 0;
   R(*acc)[32] = s_acc[warp];
-  for (int k0 = w.z; k0 < w.w; k0 += 32) {
-    const bool valid = k0 + lane < w.w;
-    const int k = valid ? k0 + lane : w.w - 1;
+  const LaneSplit ls = lane_split(lane, w.w - w.z, args.bra_ix[p0].y, args.ket_ix[w.z].y);
+  const int slot = lane / ls.t;
+  for (int k0 = w.z; k0 < w.w; k0 += 32 / ls.t) {
+    const bool valid = k0 + slot < w.w;
+    const int k = valid ? k0 + slot : w.w - 1;
     const double qk = args.ket_q[k];
     const double4 kra = args.ket_ra[k], kab = args.ket_ab[k];
     const int4 kix = args.ket_ix[k];
@@ -1289,7 +1349,7 @@ __global__ void __launch_bounds__(128, (RegMinBlocks<LA, LB, LC, LD, R,
     for (int bi = 0; bi < w.y; ++bi) {
       const int pos = bord[w.x + bi];
       const double qq = args.bra_q[pos] * qk;
-      bool act = valid && qq >= cut && (!args.same_list || k <= pos);
+      bool act = valid && ls.sub == 0 && qq >= cut && (!args.same_list || k <= pos);
       if (args.split_mode == 1) act = act && !(qq * qm < args.fp32_cut);
       else if (args.split_mode == 2) act = act && (qq * qm < args.fp32_cut);
       if (!__any_sync(0xffffffffu, act)) continue;
@@ -1335,7 +1395,7 @@ __global__ void __launch_bounds__(128, (RegMinBlocks<LA, LB, LC, LD, R,
       g.omega2 = args.omega2;
       const double sbk = (bdiag ? 0.5 : 1.0) * (kdiag ? 0.5 : 1.0) * (args.same_list && k == pos ? 0.5 : 1.0);
       R out[GB * GK * NO];
-      quartet_block_gen<LA, LB, LC, LD, R, GB, GK>(args, g, bpp, baux, bco, out, s_boys);
+      quartet_block_gen<LA, LB, LC, LD, R, GB, GK>(args, g, bpp, baux, bco, out, s_boys, ls);
       const R sR = act ? R(sbk) : R(0);
 #pragma unroll
       for (int b = 0; b < GB; ++b)
@@ -1475,17 +1535,23 @@ __global__ void __launch_bounds__(128) jk_flat_kernel(JKArgs args) {
   using CI = ClassInfo<LA, LB, LC, LD>;
   constexpr int NO = CI::NOUT;
   const int n = (int)min(*args.flat_n, (unsigned long long)args.flat_cap);
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  // a list shorter than the resident threads: groups of t lanes share its quartets
+  const int threads = gridDim.x * blockDim.x, lane = threadIdx.x & 31;
+  int t = 1;
+  while (t < 32 && (long long)n * (2 * t) <= threads) t *= 2;
+  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) / t; i < n; i += threads / t) {
     const int2 q = args.flat[i];
     if (q.x < 0) continue;   // space of a reservation that did not fit
     const BraRec br = load_bra(args, q.x);
     QuartetGeom g;
     load_quartet_rec(args, br, q.y, g);
+    const LaneSplit ls = lane_split_t(lane, t, g.npa);
     const double4* bpp = args.pp_data + g.ppa;
     const double2* baux = args.pp_aux + g.ppa;
     if constexpr (GB == 1 && GK == 1) {
       double out[NO];
-      quartet_block_reg<LA, LB, LC, LD, double>(args, g, bpp, baux, out, nullptr);
+      quartet_block_reg<LA, LB, LC, LD, double>(args, g, bpp, baux, out, nullptr, ls);
+      if (ls.sub != 0) continue;
       for (int e = 0; e < args.ndm; ++e) digest_one<LA, LB, LC, LD, double>(args, g, out, e);
     } else {
       int aoA[GB], aoB[GB], aoC[GK], aoD[GK];
@@ -1514,7 +1580,8 @@ __global__ void __launch_bounds__(128) jk_flat_kernel(JKArgs args) {
         kdiag = gx.x != 0;
       }
       double out[GB * GK * NO];
-      quartet_block_gen<LA, LB, LC, LD, double, GB, GK, true>(args, g, bpp, baux, args.pp_c + g.ppa, out, nullptr);
+      quartet_block_gen<LA, LB, LC, LD, double, GB, GK, true>(args, g, bpp, baux, args.pp_c + g.ppa, out, nullptr, ls);
+      if (ls.sub != 0) continue;
       const double sbk = (bdiag ? 0.5 : 1.0) * (kdiag ? 0.5 : 1.0) * (args.same_list && q.y == q.x ? 0.5 : 1.0);
 #pragma unroll
       for (int b = 0; b < GB; ++b)
