@@ -17,6 +17,7 @@
 // scatter (csrc/direct_jk.cc:50-75) folded by the symmetry of D.
 #pragma once
 #include "common.cuh"
+#include "os_eri.cuh"
 
 namespace b200jk {
 
@@ -368,6 +369,52 @@ __device__ __forceinline__ void lane_sum(R* v, const LaneSplit& s) {
 // Register path: one thread (or one group of lanes, above) per quartet, the
 // whole Cartesian block in registers.
 // ---------------------------------------------------------------------------
+// Which classes evaluate their primitive quartets by the Obara-Saika recursion
+// (os_eri.cuh) and which by Rys quadrature.  FP64: every class of L <= 5
+// ((H2O)32 cc-pVDZ class times: (10|10) 9.6 -> 7.7 ms, (11|10) 7.1 -> 5.9,
+// (21|10) 5.9 -> 3.8, (11|00) 5.4 -> 4.2).  FP32: only classes without a
+// horizontal transfer (l_B = l_D = 0), where it is more exact than the FP32
+// quadrature (over random quartets: (20|20) rms 1.0e-7 against 1.3e-7); the
+// transfer of the contracted block cancels leading digits that the transfer
+// of each root's one-dimensional tables keeps ((11|11) 5e-6 against 2e-6).
+template <int LA, int LB, int LC, int LD, typename R>
+struct UseOs {
+  using CI = ClassInfo<LA, LB, LC, LD>;
+  static constexpr bool value =
+      CI::NROOT <= 3 && (sizeof(R) == 4 ? LB == 0 && LD == 0 : LB <= 2 && LD <= 2);
+};
+
+// Scalars of the Obara-Saika recursion and prefactor F_m(t), m = 0..L, of one
+// primitive quartet (erf-attenuated operator: F_m -> theta^(m+1/2) F_m(theta t)).
+template <int L, typename R>
+__device__ __forceinline__ void os_setup(const JKArgs& args, const PrimQ<R>& s, const float* s_boys, OsPrim<R>& o,
+                                         R* f) {
+  o.pa[0] = s.pax; o.pa[1] = s.pay; o.pa[2] = s.paz;
+  o.qc[0] = s.qcx; o.qc[1] = s.qcy; o.qc[2] = s.qcz;
+  const R pq[3] = {s.pqx, s.pqy, s.pqz};
+#pragma unroll
+  for (int x = 0; x < 3; ++x) {
+    o.wp[x] = -s.q_pq * pq[x];
+    o.wq[x] = s.p_pq * pq[x];
+  }
+  o.inv2p = s.inv2p; o.inv2q = s.inv2q; o.inv2pq = R(0.5) * s.pq_inv;
+  o.q_pq = s.q_pq; o.p_pq = s.p_pq;
+  constexpr int N = L / 2 + 1, M = 2 * N - 1;
+  R F[M + 1];
+  if constexpr (sizeof(R) == 4) boys_fn<M, float, 10, 6>(s.t, F, s_boys);
+  else boys_fn<M, double>(s.t, F, args.tb.boys_m + (N - 1) * 801 * 8);
+#pragma unroll
+  for (int m = 0; m <= L; ++m) f[m] = F[m] * s.pref;
+  if (args.omega2 > 0.0) {
+    R th = s.theta;
+#pragma unroll
+    for (int m = 1; m <= L; ++m) {
+      f[m] *= th;
+      th *= s.theta;
+    }
+  }
+}
+
 #ifndef B200JK_REG_UNROLL
 #define B200JK_REG_UNROLL 2
 #endif
@@ -380,8 +427,11 @@ __device__ __forceinline__ void quartet_block_reg(const JKArgs& args, const Quar
   using CI = ClassInfo<LA, LB, LC, LD>;
   using GI = GIdx<LA, LB, LC, LD>;
   constexpr int N = CI::NROOT;
+  constexpr bool OS = UseOs<LA, LB, LC, LD, R>::value;
+  constexpr int NACC = OS ? OsInfo<LA, LB, LC, LD>::NACC : CI::NOUT;
+  R acc[NACC];
 #pragma unroll
-  for (int o = 0; o < CI::NOUT; ++o) out[o] = R(0);
+  for (int o = 0; o < NACC; ++o) acc[o] = R(0);
   // ket primitive in registers (outer), bra primitives broadcast from
   // shared memory (inner): one global read per ket primitive pair.
   const float3 ac = make_float3(float(g.ax - g.cx), float(g.ay - g.cy), float(g.az - g.cz));
@@ -401,6 +451,13 @@ __device__ __forceinline__ void quartet_block_reg(const JKArgs& args, const Quar
     for (int i = ls.si; i < g.npa; i += ls.ti) {
       PrimQ<R> s;
       prim_any<R>(g, ac, bpp[i], baux[i], Q, QA, s);
+      if constexpr (OS) {
+        OsPrim<R> os;
+        R f[CI::L + 1];
+        os_setup<CI::L, R>(args, s, s_boys, os, f);
+        os_vertical<LA, LB, LC, LD, R>(os, f, [&](auto O, R v) { acc[decltype(O)::value] += v; });
+        continue;
+      }
       R x[N], w[N];
       if constexpr (sizeof(R) == 4 && N <= 3)
         rys_small<N, float, 10, 6>(s.t, x, w, s_boys);   // shared-memory Taylor rows
@@ -424,12 +481,19 @@ __device__ __forceinline__ void quartet_block_reg(const JKArgs& args, const Quar
           constexpr int jx = GI::idx(cart_lx(LA, ia), cart_lx(LB, ib), cart_lx(LC, ic), cart_lx(LD, id));
           constexpr int jy = GI::idx(cart_ly(LA, ia), cart_ly(LB, ib), cart_ly(LC, ic), cart_ly(LD, id));
           constexpr int jz = GI::idx(cart_lz(LA, ia), cart_lz(LB, ib), cart_lz(LC, ic), cart_lz(LD, id));
-          out[o] += gx[jx] * gy[jy] * gz[jz];
+          if constexpr (!OS) acc[o] += gx[jx] * gy[jy] * gz[jz];
         });
       }
     }
   }
-  lane_sum<CI::NOUT>(out, ls);
+  lane_sum<NACC>(acc, ls);
+  if constexpr (OS) {
+    const R ab[3] = {R(g.abx), R(g.aby), R(g.abz)}, cd[3] = {R(g.cdx), R(g.cdy), R(g.cdz)};
+    os_horizontal<LA, LB, LC, LD, R>(acc, ab, cd, out);
+  } else {
+#pragma unroll
+    for (int o = 0; o < CI::NOUT; ++o) out[o] = acc[o];
+  }
 }
 
 // Density elements one quartet digests, in a fixed order: D[c][d] (J of the
@@ -1043,9 +1107,12 @@ __device__ __forceinline__ void quartet_block_gen(const JKArgs& args, const Quar
                                                   const float* s_boys, const LaneSplit& ls) {
   using CI = ClassInfo<LA, LB, LC, LD>;
   using GI = GIdx<LA, LB, LC, LD>;
-  constexpr int N = CI::NROOT, NO = CI::NOUT;
+  constexpr int N = CI::NROOT;
+  constexpr bool OS = UseOs<LA, LB, LC, LD, R>::value;
+  constexpr int NO = OS ? OsInfo<LA, LB, LC, LD>::NACC : CI::NOUT;
+  R acc[GB * GK * NO];
 #pragma unroll
-  for (int o = 0; o < GB * GK * NO; ++o) out[o] = R(0);
+  for (int o = 0; o < GB * GK * NO; ++o) acc[o] = R(0);
   const float3 ac = make_float3(float(g.ax - g.cx), float(g.ay - g.cy), float(g.az - g.cz));
   const int jl = g.ppc + g.npc;
   int j = min(g.ppc + ls.sj, jl - 1);
@@ -1067,14 +1134,20 @@ __device__ __forceinline__ void quartet_block_gen(const JKArgs& args, const Quar
     for (int i = ls.si; i < g.npa; i += ls.ti) {
       PrimQ<R> s;
       prim_any<R>(g, ac, bpp[i], baux[i], Q, QA, s);
+      R tmp[NO];
+#pragma unroll
+      for (int o = 0; o < NO; ++o) tmp[o] = R(0);
+      if constexpr (OS) {
+        OsPrim<R> os;
+        R f[CI::L + 1];
+        os_setup<CI::L, R>(args, s, s_boys, os, f);
+        os_vertical<LA, LB, LC, LD, R>(os, f, [&](auto O, R v) { tmp[decltype(O)::value] = v; });
+      } else {
       R x[N], w[N];
       if constexpr (sizeof(R) == 4 && N <= 3)
         rys_small<N, float, 10, 6>(s.t, x, w, s_boys);
       else
         rys_roots<N, R>(s.t, x, w, args.tb);
-      R tmp[NO];
-#pragma unroll
-      for (int o = 0; o < NO; ++o) tmp[o] = R(0);
 #pragma unroll
       for (int r = 0; r < N; ++r) {
         RootCoef<R> rc;
@@ -1086,7 +1159,7 @@ __device__ __forceinline__ void quartet_block_gen(const JKArgs& args, const Quar
                                    R(g.cdy), gy);
         build_g<LA, LB, LC, LD, R>(rc.c00[2], rc.c0p[2], rc.b10, rc.b01, rc.b00, w[r] * s.pref,
                                    R(g.abz), R(g.cdz), gz);
-        static_for<0, NO>([&](auto O) {
+        static_for<0, CI::NOUT>([&](auto O) {
           constexpr int o = decltype(O)::value;
           constexpr int id = o % CI::ND, ic = (o / CI::ND) % CI::NC;
           constexpr int ib = (o / CI::NCD) % CI::NB, ia = o / (CI::NCD * CI::NB);
@@ -1095,6 +1168,7 @@ __device__ __forceinline__ void quartet_block_gen(const JKArgs& args, const Quar
           constexpr int jz = GI::idx(cart_lz(LA, ia), cart_lz(LB, ib), cart_lz(LC, ic), cart_lz(LD, id));
           tmp[o] += gx[jx] * gy[jy] * gz[jz];
         });
+      }
       }
       const auto CB = bco[i];
       if constexpr (PRESUM) {
@@ -1112,7 +1186,7 @@ __device__ __forceinline__ void quartet_block_gen(const JKArgs& args, const Quar
             constexpr int k = decltype(KI)::value;
             const R wgt = cb * R(comp<k>(CK));
 #pragma unroll
-            for (int o = 0; o < NO; ++o) out[(b * GK + k) * NO + o] += wgt * tmp[o];
+            for (int o = 0; o < NO; ++o) acc[(b * GK + k) * NO + o] += wgt * tmp[o];
           });
         });
       }
@@ -1124,12 +1198,22 @@ __device__ __forceinline__ void quartet_block_gen(const JKArgs& args, const Quar
           constexpr int k = decltype(KI)::value;
           const R ck = R(comp<k>(CK));
 #pragma unroll
-          for (int o = 0; o < NO; ++o) out[(b * GK + k) * NO + o] += ck * sb[b * NO + o];
+          for (int o = 0; o < NO; ++o) acc[(b * GK + k) * NO + o] += ck * sb[b * NO + o];
         });
       });
     }
   }
-  lane_sum<GB * GK * NO>(out, ls);
+  lane_sum<GB * GK * NO>(acc, ls);
+#pragma unroll
+  for (int q = 0; q < GB * GK; ++q) {
+    if constexpr (OS) {
+      const R ab[3] = {R(g.abx), R(g.aby), R(g.abz)}, cd[3] = {R(g.cdx), R(g.cdy), R(g.cdz)};
+      os_horizontal<LA, LB, LC, LD, R>(acc + q * NO, ab, cd, out + q * CI::NOUT);
+    } else {
+#pragma unroll
+      for (int o = 0; o < NO; ++o) out[q * NO + o] = acc[q * NO + o];
+    }
+  }
 }
 
 template <int LA, int LB, int LC, int LD, typename R, int GB, int GK>
