@@ -504,11 +504,17 @@ def packed_jk(eri, density, *, with_j=True, with_k=True):
     real = real.to(torch.float64).contiguous()
     nops = int(bool(with_j)) + int(bool(with_k))
     out = torch.empty((nops, real.shape[0], n, n), dtype=torch.float64, device=e.device)
+    e = e.contiguous()
     with torch.cuda.device(e.device):
-        _capi.check(_capi.lib().b200jk_packed_jk(
-            ctypes.c_void_p(e.contiguous().data_ptr()), 1 if e.dim() == 1 else 0, e.numel(), n,
+        lib, nbytes = _capi.lib(), ctypes.c_int64()
+        _capi.check(lib.b200jk_packed_jk_workspace(n, real.shape[0], int(bool(with_j)), int(bool(with_k)),
+                                                   ctypes.byref(nbytes)))
+        # from torch's allocator: a buffer of this call on the current stream
+        ws = torch.empty((nbytes.value,), dtype=torch.uint8, device=e.device)
+        _capi.check(lib.b200jk_packed_jk_ws(
+            ctypes.c_void_p(e.data_ptr()), 1 if e.dim() == 1 else 0, e.numel(), n,
             ctypes.c_void_p(real.data_ptr()), real.shape[0], ctypes.c_void_p(out.data_ptr()),
-            int(bool(with_j)), int(bool(with_k)), _stream_handle()))
+            int(bool(with_j)), int(bool(with_k)), ctypes.c_void_p(ws.data_ptr()), nbytes.value, _stream_handle()))
     if d.is_complex():
         out = torch.complex(out[:, :count], out[:, count:])
     out = out.reshape(nops, *d.shape)

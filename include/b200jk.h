@@ -131,6 +131,15 @@ int b200jk_packed_jk(const double* d_eri, int32_t layout, int64_t eri_size, int3
                      const double* d_density, int32_t nb, double* d_out, int32_t with_j,
                      int32_t with_k, void* stream);
 
+/* The same on a caller-owned device workspace (16-byte aligned, at least the
+ * bytes that b200jk_packed_jk_workspace gives, its contents lost), so the call
+ * allocates nothing; b200jk_packed_jk takes its workspace from the device's
+ * stream-ordered pool instead. */
+int b200jk_packed_jk_workspace(int32_t n, int32_t nb, int32_t with_j, int32_t with_k, int64_t* bytes);
+int b200jk_packed_jk_ws(const double* d_eri, int32_t layout, int64_t eri_size, int32_t n,
+                        const double* d_density, int32_t nb, double* d_out, int32_t with_j,
+                        int32_t with_k, void* d_workspace, int64_t workspace_bytes, void* stream);
+
 /* Number of kernels one b200jk_direct_jk call launches on this plan (and
  * shard) in `precision` mode. */
 int b200jk_plan_launches(const b200jk_plan* plan, int32_t precision, int64_t* count);
