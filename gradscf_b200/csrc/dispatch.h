@@ -16,6 +16,7 @@ constexpr int kQuartetClasses = kPairClasses * (kPairClasses + 1) / 2;   // 55
 using JKLauncher = int (*)(const JKArgs&, cudaStream_t);
 using SchwarzLauncher = int (*)(const JKArgs&, int npairs, int cart, cudaStream_t);
 using GradLauncher = int (*)(const JKArgs&, cudaStream_t);
+using GeomLauncher = int (*)(const JKArgs&, int mode, cudaStream_t);   // mode 0 / 1: JVP of order 1 / 2, 2: order-2 VJP
 using StoreLauncher = int (*)(const JKArgs&, int cart, int layout, double* out, long long npair, cudaStream_t);
 
 struct DispatchTable {
@@ -25,6 +26,7 @@ struct DispatchTable {
   JKLauncher grp32[kQuartetClasses] = {};
   GradLauncher grad64[kQuartetClasses] = {};
   GradLauncher grad32[kQuartetClasses] = {};   // FP32 slice of a split-precision VJP
+  GeomLauncher geom[kQuartetClasses] = {};     // JVP and Hessian-vector products
   StoreLauncher store[kQuartetClasses] = {};   // packed ERI producer
   SchwarzLauncher schwarz[kPairClasses] = {};
   // grouped-list kernels by (bra, ket) combinations: slot 3*g(gb) + g(gk),

@@ -1721,6 +1721,37 @@ static long long jk_cost(const ClassPairWork& W) {
   return c;
 }
 
+// Independent class-pair launches spread over the caller's stream and the
+// plan's auxiliary streams (forked from and joined back into `st`):
+// longest-first onto the least-loaded stream; `serial` keeps them on `st`.
+template <typename F>
+static void spread_classes(Plan& p, cudaStream_t st, bool serial, F&& launch) {
+  const int nstreams = serial ? 1 : kAuxStreams + 1;
+  cudaStream_t streams[kAuxStreams + 1] = {st};
+  for (int i = 0; i < kAuxStreams; ++i) streams[i + 1] = p.aux[i];
+  if (!serial) {
+    CUDA_OK(cudaEventRecord(p.fork_ev, st));
+    for (int i = 0; i < kAuxStreams; ++i) CUDA_OK(cudaStreamWaitEvent(p.aux[i], p.fork_ev, 0));
+  }
+  std::vector<std::pair<long long, ClassPairWork*>> order;
+  for (auto* W : p.work)
+    if (W->nwork > 0) order.push_back({W->prim_quartets, W});
+  std::sort(order.begin(), order.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
+  std::vector<long long> load(nstreams, 0);
+  for (auto& [cost, W] : order) {
+    int best = 0;
+    for (int i = 1; i < nstreams; ++i)
+      if (load[i] < load[best]) best = i;
+    load[best] += cost;
+    launch(*W, streams[best]);
+  }
+  if (!serial)
+    for (int i = 0; i < kAuxStreams; ++i) {
+      CUDA_OK(cudaEventRecord(p.join_ev[i], p.aux[i]));
+      CUDA_OK(cudaStreamWaitEvent(st, p.join_ev[i], 0));
+    }
+}
+
 // The class-pair launches of one build spread over the caller's stream and
 // the plan's auxiliary streams (forked from and joined back into `st`): the
 // launches are independent (J/K accumulate atomically), so their tails and
@@ -2438,31 +2469,13 @@ int b200jk_direct_jk_geom_vjp_precision(b200jk_plan* plan, const double* d_densi
     a.gnb = nb;
     a.grad = d_grad;
     const auto& disp = dispatch();
-    // class pairs longest-first over the caller's and the auxiliary streams
-    // (serial while profiling, so each launch is timed alone)
-    const int nstreams = p.profiling ? 1 : kAuxStreams + 1;
-    cudaStream_t streams[kAuxStreams + 1] = {st};
-    for (int i = 0; i < kAuxStreams; ++i) streams[i + 1] = p.aux[i];
-    if (nstreams > 1) {
-      CUDA_OK(cudaEventRecord(p.fork_ev, st));
-      for (int i = 0; i < kAuxStreams; ++i) CUDA_OK(cudaStreamWaitEvent(p.aux[i], p.fork_ev, 0));
-    }
-    std::vector<std::pair<long long, ClassPairWork*>> order;
-    for (auto* W : p.work) order.push_back({W->prim_quartets, W});
-    std::sort(order.begin(), order.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
-    std::vector<long long> load(nstreams, 0);
-    for (auto& [cost, W] : order) {
-      if (W->nwork == 0) continue;
-      int best = 0;
-      for (int i = 1; i < nstreams; ++i)
-        if (load[i] < load[best]) best = i;
-      load[best] += cost;
-      cudaStream_t ls = streams[best];
-      const int cls = quartet_class(W->x, W->y);
-      set_lists(a, p, *W);
-      a.work = W->work.as<int4>();
-      a.nwork = W->nwork;
-      a.split = W->split.as<int>();
+    // serial while profiling, so each launch is timed alone
+    spread_classes(p, st, p.profiling, [&](ClassPairWork& W, cudaStream_t ls) {
+      const int cls = quartet_class(W.x, W.y);
+      set_lists(a, p, W);
+      a.work = W.work.as<int4>();
+      a.nwork = W.nwork;
+      a.split = W.split.as<int>();
       // FP64 (all kets, or the kets before each item's FP32 boundary), then the FP32 slice
       for (int slice = 0; slice < (split ? 2 : 1); ++slice) {
         a.split_mode = split ? slice + 1 : 0;
@@ -2475,37 +2488,28 @@ int b200jk_direct_jk_geom_vjp_precision(b200jk_plan* plan, const double* d_densi
         const GradLauncher lg = slice == 0 ? disp.grad64[cls] : disp.grad32[cls];
         const int rc = lg(a, ls);
         if (rc)
-          throw Failure{B200JK_INTERNAL, std::string("gradient launch failed (class pair ") + std::to_string(W->x) +
-                                             "," + std::to_string(W->y) + "): " + cudaGetErrorString((cudaError_t)rc)};
+          throw Failure{B200JK_INTERNAL, std::string("gradient launch failed (class pair ") + std::to_string(W.x) +
+                                             "," + std::to_string(W.y) + "): " + cudaGetErrorString((cudaError_t)rc)};
         if (p.profiling) {
           CUDA_OK(cudaEventRecord(ev.stop, ls));
           p.events.push_back(ev);
         }
       }
-    }
-    if (nstreams > 1)
-      for (int i = 0; i < kAuxStreams; ++i) {
-        CUDA_OK(cudaEventRecord(p.join_ev[i], p.aux[i]));
-        CUDA_OK(cudaStreamWaitEvent(st, p.join_ev[i], 0));
-      }
+    });
   });
 }
 
 // The geometry-product kernel (mode 0/1: JVP of order 1/2, 2: order-2 VJP)
 // of every class pair's expanded work items, on `a` as prepared by the caller.
 static void launch_geom_all(Plan& p, JKArgs a, int mode, cudaStream_t st) {
-  for (auto* W : p.work) {
-    if (W->nwork == 0) continue;
-    const int la = pc_la_host(W->x), lb = W->x - la * (la + 1) / 2;
-    const int lc = pc_la_host(W->y), ld = W->y - lc * (lc + 1) / 2;
-    if (!geom_smem_bytes(la, lb, lc, ld)) throw Failure{B200JK_UNSUPPORTED, "class too large for the geometry products"};
-    set_lists(a, p, *W);
-    a.work = W->work.as<int4>();
-    a.nwork = W->nwork;
-    a.split_mode = 0;
-    const int rc = launch_geom(a, la, lb, lc, ld, mode, st);
+  a.split_mode = 0;
+  spread_classes(p, st, false, [&](ClassPairWork& W, cudaStream_t ls) {
+    set_lists(a, p, W);
+    a.work = W.work.as<int4>();
+    a.nwork = W.nwork;
+    const int rc = dispatch().geom[quartet_class(W.x, W.y)](a, mode, ls);
     if (rc) throw Failure{B200JK_INTERNAL, std::string("geometry product launch failed: ") + cudaGetErrorString((cudaError_t)rc)};
-  }
+  });
 }
 
 int b200jk_direct_jk_geom_jvp(b200jk_plan* plan, const double* d_density, int32_t nb, int32_t hermi,

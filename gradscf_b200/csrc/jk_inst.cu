@@ -4,6 +4,7 @@
 #include <algorithm>
 
 #include "dispatch.h"
+#include "geom_kernels.cuh"
 #include "grad_kernels.cuh"
 #include "jk_kernels.cuh"
 
@@ -218,6 +219,21 @@ int launch_grad(const JKArgs& args, cudaStream_t stream) {
   return (int)cudaGetLastError();
 }
 
+// The geometry products of one class pair: a block per (item, ket stride);
+// items split over gridDim.y blocks until the launch holds about four blocks
+// per resident one (148 x 3 at 64 KB).
+template <int LA, int LB, int LC, int LD>
+int launch_geom(const JKArgs& args, int mode, cudaStream_t stream) {
+  if (args.nwork <= 0) return 0;
+  constexpr size_t smem = GeoCfg<LA, LB, LC, LD>::bytes();
+  static std::atomic<uint64_t> smem_done{0};
+  const cudaError_t ea = smem_opt_in(geom_kernel<LA, LB, LC, LD>, smem, smem_done);
+  if (ea != cudaSuccess) return (int)ea;
+  const int gy = std::min(32, std::max(1, 1776 / args.nwork));
+  geom_kernel<LA, LB, LC, LD><<<dim3(args.nwork, gy), kGeoThreads, smem, stream>>>(args, mode);
+  return (int)cudaGetLastError();
+}
+
 constexpr int X = BRA_CLASS;
 constexpr int Y = KET_CLASS;
 static_assert(Y <= X, "ket class must not exceed bra class");
@@ -278,6 +294,7 @@ void REG_NAME(BRA_CLASS, KET_CLASS)(DispatchTable& t) {
   }
   t.grad64[id] = &launch_grad<XA, XB, YA, YB, double>;
   t.grad32[id] = &launch_grad<XA, XB, YA, YB, float>;
+  t.geom[id] = &launch_geom<XA, XB, YA, YB>;
   t.store[id] = &launch_store<XA, XB, YA, YB>;
   t.reg_path[id] = Policy<XA, XB, YA, YB, float>::REG || Policy<XA, XB, YA, YB>::REG;
   t.tile[id] = Policy<XA, XB, YA, YB>::TILE;

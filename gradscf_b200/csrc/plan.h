@@ -205,10 +205,6 @@ void run_jk_core(Plan& p, const double* d_in, int nb, double* d_out, int with_j,
                  int hermi, int precision, double fp32_cut, cudaStream_t st, double* s_dens,
                  float* s_dens_f, double* s_vj, double* s_vk, bool allow_profiling);
 int guarded_call(const std::function<void()>& f);
-// coordinate JVP (mode 0: order 1, 1: order 2) and order-2 VJP (mode 2) of
-// one class pair's expanded work items (geom.cu)
-int launch_geom(const JKArgs& args, int la, int lb, int lc, int ld, int mode, cudaStream_t st);
-size_t geom_smem_bytes(int la, int lb, int lc, int ld);
 void fail_invalid(const std::string& m);
 
 // Device-wide constant tables (Rys, Boys, c2s) of the current device.
