@@ -97,8 +97,9 @@ struct Tables {
   // (double) / 32-byte (float) row per lookup.
   const double* boys_m;
   const float* boys_m_f;
-  // FP32 copies at spacing 1/10 (401 rows of 8, terms F_{M+i}/i!), staged in
-  // shared memory by the FP32 register path.
+  // FP32 copies of the first four terms (801 rows of 4, one 16-byte load per
+  // lookup), staged in shared memory by the FP32 register path: at spacing
+  // 1/20 the fifth term is below 0.025^4 / 24 = 1.6e-8 of F_{M+4}.
   const float* boys_s_f;
 };
 
@@ -117,13 +118,17 @@ constexpr int kTS = kTW * kTW;
 // Division-free: constant divisors are multiplications by folded reciprocals.
 template <int M, typename R, int SINV = 20, int NT = (sizeof(R) == 8 ? 8 : 5)>
 __device__ __forceinline__ void boys_fn(R t, R* f, const R* tab) {
-  // tab: this order's table, rows of 8 at spacing 1/SINV over [0, 40]
+  // tab: this order's table, rows of 8 (of 4 for NT <= 4) at spacing 1/SINV over [0, 40]
+  constexpr int ROW = NT <= 4 ? 4 : 8;
   if (t < R(40)) {
     const int k = min(max(__float2int_rn(float(t) * float(SINV)), 0), 40 * SINV);
     const R dt = R(k) * R(1.0 / SINV) - t;          // -(t - t_k)
-    const R* row = tab + k * 8;
+    const R* row = tab + k * ROW;
     R c[8];
-    if constexpr (sizeof(R) == 8) {
+    if constexpr (ROW == 4) {
+      const float4 a = *reinterpret_cast<const float4*>(row);
+      c[0] = a.x; c[1] = a.y; c[2] = a.z; c[3] = a.w;
+    } else if constexpr (sizeof(R) == 8) {
       const double4 a = reinterpret_cast<const double4*>(row)[0];
       const double4 b = reinterpret_cast<const double4*>(row)[1];
       c[0] = a.x; c[1] = a.y; c[2] = a.z; c[3] = a.w; c[4] = b.x; c[5] = b.y; c[6] = b.z; c[7] = b.w;

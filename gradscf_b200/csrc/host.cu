@@ -133,10 +133,9 @@ static DeviceTables& tables_for(int device) {
         }
       }
     up(d->boys_m, bm.data(), bm.size() * sizeof(double));
-    std::vector<float> bs(3 * 401 * 8);
-    for (int mi = 0; mi < 3; ++mi)
-      for (int k = 0; k < 401; ++k)
-        for (int i = 0; i < 8; ++i) bs[(mi * 401 + k) * 8 + i] = float(bm[(mi * 801 + 2 * k) * 8 + i]);
+    std::vector<float> bs(3 * 801 * 4);
+    for (int r = 0; r < 3 * 801; ++r)
+      for (int i = 0; i < 4; ++i) bs[r * 4 + i] = float(bm[r * 8 + i]);
     up(d->boys_s_f, bs.data(), bs.size() * sizeof(float));
     std::vector<float> bmf(bm.begin(), bm.end());
     up(d->boys_m_f, bmf.data(), bmf.size() * sizeof(float));

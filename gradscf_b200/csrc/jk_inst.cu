@@ -102,7 +102,7 @@ int launch_grp(const JKArgs& args, cudaStream_t stream) {
 template <int LA, int LB, int LC, int LD, typename R, int GB, int GK>
 int launch_grp_gen(const JKArgs& args, cudaStream_t stream) {
   if (args.nwork <= 0) return 0;
-  constexpr size_t smem = (size_t)kRegWarps * GrpGenAcc<LA, LB, LC, LD, GB, GK>::N * 32 * sizeof(R);
+  constexpr size_t smem = GrpGenAcc<LA, LB, LC, LD, GB, GK>::template bytes<R>();
   // static caches plus these pass sums pass 48 KB for most buckets: opt in
   // (to at least 64 KB of dynamic shared memory) for every one
   static std::atomic<uint64_t> smem_done{0};
