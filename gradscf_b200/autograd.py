@@ -74,9 +74,14 @@ class _DirectJK(torch.autograd.Function):
         gk = torch.zeros_like(d) if gk is None else gk.contiguous()
         grad_d = grad_c = None
         if ctx.needs_input_grad[0]:
-            jj, _ = _jk(plan, gj, False, basis.precision, basis.fp32_cut)
-            _, kk = _jk(plan, gk, False, basis.precision, basis.fp32_cut)
-            grad_d = jj + kk
+            # J sees the symmetric part of its density only; K of a symmetric
+            # cotangent needs no antisymmetric set
+            n2 = plan.nao[0] ** 2
+            opts = dict(precision=basis.precision, fp32_cut=basis.fp32_cut)
+            grad_d = plan.jk_packed(gj.reshape(-1, n2), with_k=False, hermi=1, **opts)[0]
+            hermi = bool(torch.equal(gk, gk.transpose(-1, -2)))
+            grad_d = grad_d + plan.jk_packed(gk.reshape(-1, n2), with_j=False, hermi=hermi, **opts)[0]
+            grad_d = grad_d.reshape(d.shape)
         if ctx.needs_input_grad[1]:
             n = plan.nao[0]
             nb = d.numel() // (n * n)
