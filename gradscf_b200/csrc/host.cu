@@ -2380,15 +2380,13 @@ int b200jk_packed_eri(b200jk_plan* plan, int32_t layout, double* d_out, int64_t 
     CUDA_OK(cudaMemsetAsync(d_out, 0, (size_t)size * sizeof(double), st));
     JKArgs a = base_args(p);
     const auto& disp = dispatch();
-    for (auto* W : p.work) {
-      if (W->nwork == 0) continue;
-      const int cls = quartet_class(W->x, W->y);
-      set_lists(a, p, *W);
-      a.work = W->work.as<int4>();
-      a.nwork = W->nwork;
-      const int rc = disp.store[cls](a, p.cart, layout, d_out, np, st);
+    spread_classes(p, st, false, [&](ClassPairWork& W, cudaStream_t ls) {
+      set_lists(a, p, W);
+      a.work = W.work.as<int4>();
+      a.nwork = W.nwork;
+      const int rc = disp.store[quartet_class(W.x, W.y)](a, p.cart, layout, d_out, np, ls);
       if (rc) throw Failure{B200JK_INTERNAL, std::string("packed ERI launch failed: ") + cudaGetErrorString((cudaError_t)rc)};
-    }
+    });
   });
 }
 

@@ -74,6 +74,10 @@ int launch_class(const JKArgs& args, cudaStream_t stream) {
 template <int LA, int LB, int LC, int LD>
 int launch_store(const JKArgs& args, int cart, int layout, double* out, long long npair, cudaStream_t stream) {
   if (args.nwork <= 0) return 0;
+  if constexpr (Policy<LA, LB, LC, LD>::REG) {
+    eri_reg_kernel<LA, LB, LC, LD><<<(args.nwork + 3) / 4, 128, 0, stream>>>(args, cart, layout, out, npair);
+    return (int)cudaGetLastError();
+  } else {
   using CI = ClassInfo<LA, LB, LC, LD>;
   constexpr int TEAM = Policy<LA, LB, LC, LD>::TEAM;
   using SM = TeamSmem<LA, LB, LC, LD, double, TEAM>;
@@ -85,6 +89,7 @@ int launch_store(const JKArgs& args, int cart, int layout, double* out, long lon
   smem_opt_in(eri_store_kernel<LA, LB, LC, LD, TEAM>, smem, smem_done);
   eri_store_kernel<LA, LB, LC, LD, TEAM><<<args.nwork, teams * TEAM, smem, stream>>>(args, cart, layout, out, npair);
   return (int)cudaGetLastError();
+  }
 }
 
 // Persistent launches of the bra-group kernels: at most one wave of resident
@@ -140,6 +145,10 @@ int launch_gen(const JKArgs& args, cudaStream_t stream) {
 template <int LA, int LB>
 int launch_schwarz(const JKArgs& args, int npairs, int cart, cudaStream_t stream) {
   if (npairs <= 0) return 0;
+  if constexpr (Policy<LA, LB, LA, LB>::REG) {
+    schwarz_reg_kernel<LA, LB><<<(npairs + 3) / 4, 128, 0, stream>>>(args, npairs, cart);
+    return (int)cudaGetLastError();
+  } else {
   constexpr int TEAM = Policy<LA, LB, LA, LB>::TEAM;
   using SM = TeamSmem<LA, LB, LA, LB, double, TEAM>;
   constexpr size_t per_team = SM::bytes();
@@ -151,6 +160,7 @@ int launch_schwarz(const JKArgs& args, int npairs, int cart, cudaStream_t stream
   const int blocks = (npairs + teams - 1) / teams;
   schwarz_kernel<LA, LB, TEAM><<<blocks, teams * TEAM, smem, stream>>>(args, npairs, cart);
   return (int)cudaGetLastError();
+  }
 }
 #endif
 

@@ -2106,6 +2106,49 @@ __global__ void schwarz_kernel(JKArgs args, int npairs, int cart) {
   if (lane == 0) args.q_out[pair] = best;
 }
 
+// The same for the classes whose diagonal block fits the registers: a warp
+// per pair, its lanes sharing the pair's primitive quartets (the oxygen core
+// pair has 4096; on the team path four lanes walked them one by one: 2.1 ms of
+// every plan with an oxygen).
+template <int LA, int LB>
+__global__ void __launch_bounds__(128) schwarz_reg_kernel(JKArgs args, int npairs, int cart) {
+  using CI = ClassInfo<LA, LB, LA, LB>;
+  __shared__ double s_v[4][CI::NOUT];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, pos = blockIdx.x * 4 + warp;
+  if (pos >= npairs) return;
+  const int pair = args.bra_pairs[pos];
+  QuartetGeom g;
+  load_quartet(args, pair, pair, g);
+  const LaneSplit ls = lane_split_t(lane, 32, g.npa);
+  double out[CI::NOUT];
+  quartet_block_reg<LA, LB, LA, LB, double>(args, g, args.pp_data + g.ppa, args.pp_aux + g.ppa, out, nullptr, ls);
+  double* V = s_v[warp];
+  if (lane == 0) {
+#pragma unroll
+    for (int o = 0; o < CI::NOUT; ++o) V[o] = out[o];
+  }
+  __syncwarp();
+  const int nfa = cart ? CI::NA : 2 * LA + 1, nfb = cart ? CI::NB : 2 * LB + 1;
+  const double* ta = args.tb.c2s + LA * kTS;
+  const double* tb = args.tb.c2s + LB * kTS;
+  double best = 0.0;
+  for (int t = lane; t < nfa * nfb; t += 32) {
+    const int fa = t / nfb, fb = t % nfb;
+    double acc = 0.0;
+    for (int a1 = 0; a1 < CI::NA; ++a1)
+      for (int b1 = 0; b1 < CI::NB; ++b1) {
+        const double x1 = ta[a1 * kTW + fa] * tb[b1 * kTW + fb];
+        if (x1 == 0.0) continue;
+        for (int a2 = 0; a2 < CI::NA; ++a2)
+          for (int b2 = 0; b2 < CI::NB; ++b2)
+            acc += x1 * ta[a2 * kTW + fa] * tb[b2 * kTW + fb] * V[((a1 * CI::NB + b1) * CI::NA + a2) * CI::NB + b2];
+      }
+    best = fmax(best, fabs(acc));
+  }
+  for (int off = 16; off > 0; off >>= 1) best = fmax(best, __shfl_down_sync(0xffffffffu, best, off));
+  if (lane == 0) args.q_out[pair] = best;
+}
+
 }  // namespace b200jk
 
 namespace b200jk {
@@ -2201,6 +2244,90 @@ __global__ void eri_store_kernel(JKArgs args, int cart, int layout, double* __re
       }
     }
     __syncwarp(mask);
+  }
+}
+
+// The producer for the classes on the register path: a warp per item, one
+// quartet per lane or group of lanes (lane_split), the contracted Cartesian
+// block in registers.  Shells up to p (and Cartesian output) transform by one
+// factor per shell, so their blocks go to memory from the registers; blocks
+// with spherical d or f shells are transformed quartet by quartet through
+// shared memory by the whole warp.  (H2O)4 cc-pVDZ s8: 11.0 -> 1.39 ms.
+template <int LA, int LB, int LC, int LD>
+__global__ void __launch_bounds__(128) eri_reg_kernel(JKArgs args, int cart, int layout, double* __restrict__ out,
+                                                      long long npair) {
+  using CI = ClassInfo<LA, LB, LC, LD>;
+  constexpr int NO = CI::NOUT;
+  constexpr bool kPlain = LA <= 1 && LB <= 1 && LC <= 1 && LD <= 1;
+  __shared__ double s_v[kPlain ? 1 : 8][NO];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, item = blockIdx.x * 4 + warp;
+  if (item >= args.nwork) return;
+  const int4 w = args.work[item];
+  const BraRec br = load_bra(args, w.x);
+  const int4 bp = args.pair_info[args.bra_pairs[w.x]];
+  const int oA = args.sh_info[bp.x].w, oB = args.sh_info[bp.y].w;
+  const int ls_[4] = {LA, LB, LC, LD};
+  double scale = 1.0;   // the shells whose transform is one factor
+  for (int x = 0; x < 4; ++x)
+    if (cart || ls_[x] <= 1) scale *= args.tb.c2s[ls_[x] * kTS];
+  const LaneSplit ls = lane_split(lane, w.z - w.y, br.ix.y, args.ket_ix[w.y].y);
+  const int slot = lane / ls.t, per = 32 / ls.t;
+  auto put = [&](int a, int b, int c, int d, double v) {
+    const long long ab = pair_idx(a, b), cd = pair_idx(c, d);
+    if (layout == 0) {
+      out[ab * npair + cd] = v;
+      out[cd * npair + ab] = v;
+    } else {
+      out[pair_idx(ab, cd)] = v;
+    }
+  };
+  for (int k0 = w.y; k0 < w.z; k0 += per) {
+    const bool active = k0 + slot < w.z;
+    const int k = active ? k0 + slot : w.z - 1;
+    QuartetGeom g;
+    load_quartet_rec(args, br, k, g);
+    const int4 kp = args.pair_info[args.ket_pairs[k]];
+    const int oC = args.sh_info[kp.x].w, oD = args.sh_info[kp.y].w;
+    double blk[NO];
+    quartet_block_reg<LA, LB, LC, LD, double>(args, g, args.pp_data + g.ppa, args.pp_aux + g.ppa, blk, nullptr, ls);
+    if (kPlain || cart) {
+      if (active && ls.sub == 0) {
+        static_for_n<NO>([&](auto O) {
+          constexpr int o = decltype(O)::value;
+          constexpr int id = o % CI::ND, ic = (o / CI::ND) % CI::NC;
+          constexpr int ib = (o / CI::NCD) % CI::NB, ia = o / (CI::NCD * CI::NB);
+          put(oA + ia, oB + ib, oC + ic, oD + id, scale * blk[o]);
+        });
+      }
+    } else if constexpr (!kPlain) {
+      double *src = s_v[2 * warp], *dst = s_v[2 * warp + 1];
+      for (int q = 0; q < per && k0 + q < w.z; ++q) {
+        const int from = q * ls.t;
+        __syncwarp();
+        if (lane == from) {
+          static_for_n<NO>([&](auto O) { src[decltype(O)::value] = scale * blk[decltype(O)::value]; });
+        }
+        const int qc = __shfl_sync(0xffffffffu, oC, from), qd = __shfl_sync(0xffffffffu, oD, from);
+        __syncwarp();
+        int dims[4] = {CI::NA, CI::NB, CI::NC, CI::ND};
+        double *x = src, *y = dst;
+        for (int axis = 3; axis >= 0; --axis) {
+          const int l = ls_[axis];
+          if (l <= 1) continue;
+          transform_axis(x, y, dims, axis, args.tb.c2s + l * kTS, 2 * l + 1, lane, 32);
+          __syncwarp();
+          dims[axis] = 2 * l + 1;
+          double* t = x;
+          x = y;
+          y = t;
+        }
+        const int total = dims[0] * dims[1] * dims[2] * dims[3];
+        for (int e = lane; e < total; e += 32) {
+          const int fd = e % dims[3], fc = (e / dims[3]) % dims[2], fb = (e / (dims[3] * dims[2])) % dims[1];
+          put(oA + e / (dims[3] * dims[2] * dims[1]), oB + fb, qc + fc, qd + fd, x[e]);
+        }
+      }
+    }
   }
 }
 
