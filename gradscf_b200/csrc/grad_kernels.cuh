@@ -6,25 +6,17 @@
 // all n^4 entries instead).  Derivatives recomputed, never stored:
 //   d/dA_x phi_a = 2 alpha phi_{a+1x} - a_x phi_{a-1x}  (same for B, C),
 //   d/dD = -(d/dA + d/dB + d/dC)  (translational invariance).
-// Team layout as the J/K team path: 2D integrals with raised bra/ket
-// indices in shared memory, each lane owns a strided slice of the Cartesian
-// block, nine gradient partials per lane reduced across the team.
+// Three kernels by block size: grad_reg_kernel and grad_lane_kernel (one lane
+// per quartet), grad_unit_kernel (a warp or a block per quartet).
 #pragma once
 #include "jk_kernels.cuh"
 
 namespace b200jk {
 
-template <int LA, int LB, int LC, int LD, int TEAM>
+// Roots of a first-derivative quartet.
+template <int LA, int LB, int LC, int LD>
 struct GradCfg {
-  using CI = ClassInfo<LA, LB, LC, LD>;
-  static constexpr int NROOT = (CI::L + 1) / 2 + 1;
-  static constexpr int NG = (LA + 2) * (LB + 2) * (LC + 2) * (LD + 1);
-  static constexpr int NK = (CI::NOUT + TEAM - 1) / TEAM;
-  static constexpr int ELEMS = 3 * NROOT * NG + 2 * NROOT;
-  static constexpr size_t bytes() { return (size_t)ELEMS * 8; }
-  __host__ __device__ static constexpr int idx(int a, int b, int c, int d) {
-    return ((a * (LB + 2) + b) * (LC + 2) + c) * (LD + 1) + d;
-  }
+  static constexpr int NROOT = (LA + LB + LC + LD + 1) / 2 + 1;
 };
 
 // Raw Cartesian Gamma of one AO quartet (a, b, c, d), summed over batches.
@@ -69,255 +61,9 @@ __device__ __forceinline__ void grad_prim(const JKArgs& args, const QuartetGeom&
               PrimData<R>::b(args, j), s);
 }
 
-template <int LA, int LB, int LC, int LD, int TEAM, typename R>
-__global__ void grad_team_kernel(JKArgs args) {
-  using CI = ClassInfo<LA, LB, LC, LD>;
-  using GC = GradCfg<LA, LB, LC, LD, TEAM>;
-  constexpr int N = GC::NROOT;
-  constexpr int NG = GC::NG;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int lane = threadIdx.x % TEAM;
-  const int team = threadIdx.x / TEAM;
-  const int nteams = blockDim.x / TEAM;
-  const unsigned mask =
-      TEAM == 32 ? 0xffffffffu : (((1u << TEAM) - 1u) << ((threadIdx.x % 32) / TEAM * TEAM));
-  R* G = reinterpret_cast<R*>(smem_raw) + (size_t)team * GC::ELEMS;
-  R* roots = G + 3 * N * NG;
-  const int4 w = args.work[blockIdx.x];
-  const int bra = args.bra_pairs[w.x];
-  int kb, ke;
-  grad_ket_range(args, blockIdx.x, w, kb, ke);
-  for (int k = kb + team; k < ke; k += nteams) {
-    QuartetGeom g;
-    load_quartet(args, bra, args.ket_pairs[k], g);
-    const long long base = args.mol_base[g.mol];
-    const int n = args.mol_n[g.mol];
-    R gam[GC::NK];
-    int exps[GC::NK];   // packed exponent digits of (a, b, c, d) per axis
-#pragma unroll
-    for (int q = 0; q < GC::NK; ++q) {
-      const int o = lane + q * TEAM;
-      gam[q] = R(0);
-      exps[q] = -1;
-      if (o < CI::NOUT) {
-        const int id = o % CI::ND, ic = (o / CI::ND) % CI::NC;
-        const int ib = (o / CI::NCD) % CI::NB, ia = o / (CI::NCD * CI::NB);
-        gam[q] = R(g.scale * gamma_abcd(args, base, n, g.aoA + ia, g.aoB + ib, g.aoC + ic, g.aoD + id));
-        exps[q] = ia | (ib << 4) | (ic << 8) | (id << 12);
-      }
-    }
-    R dA[3] = {0, 0, 0}, dB[3] = {0, 0, 0}, dC[3] = {0, 0, 0};
-    for (int i = g.ppa; i < g.ppa + g.npa; ++i) {
-      const R alpha = R(args.pp_exp[i].x), beta = R(args.pp_exp[i].y);
-      for (int j = g.ppc; j < g.ppc + g.npc; ++j) {
-        PrimQ<R> s;
-        grad_prim<R>(args, g, i, j, s);
-        const R gamma_c = R(args.pp_exp[j].x);
-        for (int f = lane; f < 2 * N; f += TEAM) roots[f] = rys_one<N, R>(s.t, f, args.tb);
-        __syncwarp(mask);
-        for (int tsk = lane; tsk < 3 * N; tsk += TEAM) {
-          const int r = tsk / 3, ax = tsk - 3 * r;
-          RootCoef<R> rc;
-          root_coef<R>(s, roots[r], rc);
-          const R abd = R(ax == 0 ? g.abx : (ax == 1 ? g.aby : g.abz));
-          const R cdd = R(ax == 0 ? g.cdx : (ax == 1 ? g.cdy : g.cdz));
-          const R g00 = ax == 2 ? roots[N + r] * s.pref : R(1);
-          build_g<LA + 1, LB + 1, LC + 1, LD, R>(rc.c00[ax], rc.c0p[ax], rc.b10, rc.b01, rc.b00, g00, abd, cdd,
-                                                 G + (r * 3 + ax) * NG);
-        }
-        __syncwarp(mask);
-#pragma unroll
-        for (int q = 0; q < GC::NK; ++q) {
-          if (exps[q] < 0 || gam[q] == R(0)) continue;
-          const int ia = exps[q] & 15, ib = (exps[q] >> 4) & 15, ic = (exps[q] >> 8) & 15, id = exps[q] >> 12;
-          const int la[3] = {cart_lx(LA, ia), cart_ly(LA, ia), cart_lz(LA, ia)};
-          const int lb[3] = {cart_lx(LB, ib), cart_ly(LB, ib), cart_lz(LB, ib)};
-          const int lc[3] = {cart_lx(LC, ic), cart_ly(LC, ic), cart_lz(LC, ic)};
-          const int ld[3] = {cart_lx(LD, id), cart_ly(LD, id), cart_lz(LD, id)};
-          for (int r = 0; r < N; ++r) {
-            R v[3], fa[3], fb[3], fc[3];
-#pragma unroll
-            for (int x = 0; x < 3; ++x) {
-              const R* Gx = G + (r * 3 + x) * NG;
-              const int a = la[x], b = lb[x], c = lc[x], d = ld[x];
-              v[x] = Gx[GC::idx(a, b, c, d)];
-              fa[x] = R(2) * alpha * Gx[GC::idx(a + 1, b, c, d)] - (a ? R(a) * Gx[GC::idx(a - 1, b, c, d)] : R(0));
-              fb[x] = R(2) * beta * Gx[GC::idx(a, b + 1, c, d)] - (b ? R(b) * Gx[GC::idx(a, b - 1, c, d)] : R(0));
-              fc[x] = R(2) * gamma_c * Gx[GC::idx(a, b, c + 1, d)] - (c ? R(c) * Gx[GC::idx(a, b, c - 1, d)] : R(0));
-            }
-            const R gq = gam[q];
-            const R yz = v[1] * v[2], xz = v[0] * v[2], xy = v[0] * v[1];
-            dA[0] += gq * fa[0] * yz; dA[1] += gq * fa[1] * xz; dA[2] += gq * fa[2] * xy;
-            dB[0] += gq * fb[0] * yz; dB[1] += gq * fb[1] * xz; dB[2] += gq * fb[2] * xy;
-            dC[0] += gq * fc[0] * yz; dC[1] += gq * fc[1] * xz; dC[2] += gq * fc[2] * xy;
-          }
-        }
-        __syncwarp(mask);
-      }
-    }
-    // reduce the nine partials over the team; lane 0 adds to the four centres
-#pragma unroll
-    for (int x = 0; x < 3; ++x)
-#pragma unroll
-      for (int off = TEAM / 2; off > 0; off >>= 1) {
-        dA[x] += __shfl_down_sync(mask, dA[x], off, TEAM);
-        dB[x] += __shfl_down_sync(mask, dB[x], off, TEAM);
-        dC[x] += __shfl_down_sync(mask, dC[x], off, TEAM);
-      }
-    if (lane == 0) {
-      double* gA = args.grad + 3LL * args.ws_atm[g.A];
-      double* gB = args.grad + 3LL * args.ws_atm[g.B];
-      double* gC = args.grad + 3LL * args.ws_atm[g.C];
-      double* gD = args.grad + 3LL * args.ws_atm[g.D];
-#pragma unroll
-      for (int x = 0; x < 3; ++x) {
-        atomicAdd(gA + x, double(dA[x]));
-        atomicAdd(gB + x, double(dB[x]));
-        atomicAdd(gC + x, double(dC[x]));
-        atomicAdd(gD + x, -(double(dA[x]) + double(dB[x]) + double(dC[x])));
-      }
-    }
-  }
-}
-
 }  // namespace b200jk
 
 namespace b200jk {
-
-// ---------------------------------------------------------------------------
-// Block-wide coordinate VJP for the large classes (NOUT > 256, i.e. d and f
-// shells): the whole block works on one quartet at a time.  Gamma of every
-// element is staged in shared memory once per quartet; per primitive
-// quartet the raised 2D tables of every root and axis are built in shared
-// memory (build_g_mem, one thread per table, recursion scratch in shared
-// memory so the kernel's register count stays that of the accumulation);
-// the threads then stride over the elements, each summing the nine centre
-// partials, which are block-reduced per quartet.
-// ---------------------------------------------------------------------------
-template <int LA, int LB, int LC, int LD>
-struct GradBlk {
-  using CI = ClassInfo<LA, LB, LC, LD>;
-  using GC = GradCfg<LA, LB, LC, LD, 1>;
-  static constexpr int THREADS = 128;
-  static constexpr int N = GC::NROOT, NG = GC::NG;
-  static constexpr int LAB = LA + LB + 2, LCD = LC + LD + 1;
-  static constexpr int NW = (LAB + 1) * (LCD + 1) * (LD + 1);   // recursion scratch per table
-  static constexpr int G_OFF = 0, R_OFF = 3 * N * NG, W_OFF = R_OFF + 2 * N, GAM_OFF = W_OFF + 3 * N * NW;
-  static constexpr int ELEMS = GAM_OFF + CI::NOUT;
-  static constexpr size_t bytes() { return (size_t)ELEMS * 8; }   // FP64; FP32 takes half
-  static constexpr bool OK = CI::NOUT > 256 && bytes() <= 220 * 1024;
-};
-
-template <int LA, int LB, int LC, int LD, typename R>
-__global__ void __launch_bounds__(128) grad_block_kernel(JKArgs args) {
-  using CI = ClassInfo<LA, LB, LC, LD>;
-  using GB = GradBlk<LA, LB, LC, LD>;
-  using GC = GradCfg<LA, LB, LC, LD, 1>;
-  constexpr int N = GB::N, NG = GB::NG;
-  extern __shared__ __align__(16) unsigned char gsm_raw[];
-  R* gsm = reinterpret_cast<R*>(gsm_raw);
-  R* G = gsm + GB::G_OFF;
-  R* roots = gsm + GB::R_OFF;
-  R* scratch = gsm + GB::W_OFF;
-  R* gam = gsm + GB::GAM_OFF;
-  __shared__ double red[9][GB::THREADS / 32];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int4 w = args.work[blockIdx.x];
-  const int bra = args.bra_pairs[w.x];
-  int kb, ke;
-  grad_ket_range(args, blockIdx.x, w, kb, ke);
-  for (int k = kb; k < ke; ++k) {
-    QuartetGeom g;
-    load_quartet(args, bra, args.ket_pairs[k], g);
-    const long long base = args.mol_base[g.mol];
-    const int n = args.mol_n[g.mol];
-    for (int o = tid; o < CI::NOUT; o += GB::THREADS) {
-      const int id = o % CI::ND, ic = (o / CI::ND) % CI::NC;
-      const int ib = (o / CI::NCD) % CI::NB, ia = o / (CI::NCD * CI::NB);
-      gam[o] = R(g.scale * gamma_abcd(args, base, n, g.aoA + ia, g.aoB + ib, g.aoC + ic, g.aoD + id));
-    }
-    R dA[3] = {0, 0, 0}, dB[3] = {0, 0, 0}, dC[3] = {0, 0, 0};
-    for (int i = g.ppa; i < g.ppa + g.npa; ++i) {
-      const R alpha = R(args.pp_exp[i].x), beta = R(args.pp_exp[i].y);
-      for (int j = g.ppc; j < g.ppc + g.npc; ++j) {
-        PrimQ<R> s;
-        grad_prim<R>(args, g, i, j, s);
-        const R gamma_c = R(args.pp_exp[j].x);
-        __syncthreads();   // the previous primitive quartet's tables are no longer read
-        if (tid < 2 * N) roots[tid] = rys_one<N, R>(s.t, tid, args.tb);
-        __syncthreads();
-        if (tid < 3 * N) {
-          const int r = tid / 3, ax = tid - 3 * r;
-          RootCoef<R> rc;
-          root_coef<R>(s, roots[r], rc);
-          const R abd = R(ax == 0 ? g.abx : (ax == 1 ? g.aby : g.abz));
-          const R cdd = R(ax == 0 ? g.cdx : (ax == 1 ? g.cdy : g.cdz));
-          const R g00 = ax == 2 ? roots[N + r] * s.pref : R(1);
-          build_g_mem<LA + 1, LB + 1, LC + 1, LD, R>(rc.c00[ax], rc.c0p[ax], rc.b10, rc.b01, rc.b00, g00, abd, cdd,
-                                                    G + tid * NG, scratch + tid * GB::NW);
-        }
-        __syncthreads();
-        for (int o = tid; o < CI::NOUT; o += GB::THREADS) {
-          const R gq = gam[o];
-          if (gq == R(0)) continue;
-          const int id = o % CI::ND, ic = (o / CI::ND) % CI::NC;
-          const int ib = (o / CI::NCD) % CI::NB, ia = o / (CI::NCD * CI::NB);
-          const int la[3] = {cart_lx(LA, ia), cart_ly(LA, ia), cart_lz(LA, ia)};
-          const int lb[3] = {cart_lx(LB, ib), cart_ly(LB, ib), cart_lz(LB, ib)};
-          const int lc[3] = {cart_lx(LC, ic), cart_ly(LC, ic), cart_lz(LC, ic)};
-          const int ld[3] = {cart_lx(LD, id), cart_ly(LD, id), cart_lz(LD, id)};
-#pragma unroll 2
-          for (int r = 0; r < N; ++r) {
-            R v[3], fa[3], fb[3], fc[3];
-#pragma unroll
-            for (int x = 0; x < 3; ++x) {
-              const R* Gx = G + (r * 3 + x) * NG;
-              const int a = la[x], b = lb[x], c = lc[x], d = ld[x];
-              v[x] = Gx[GC::idx(a, b, c, d)];
-              fa[x] = R(2) * alpha * Gx[GC::idx(a + 1, b, c, d)] - (a ? R(a) * Gx[GC::idx(a - 1, b, c, d)] : R(0));
-              fb[x] = R(2) * beta * Gx[GC::idx(a, b + 1, c, d)] - (b ? R(b) * Gx[GC::idx(a, b - 1, c, d)] : R(0));
-              fc[x] = R(2) * gamma_c * Gx[GC::idx(a, b, c + 1, d)] - (c ? R(c) * Gx[GC::idx(a, b, c - 1, d)] : R(0));
-            }
-            const R yz = gq * v[1] * v[2], xz = gq * v[0] * v[2], xy = gq * v[0] * v[1];
-            dA[0] += fa[0] * yz; dA[1] += fa[1] * xz; dA[2] += fa[2] * xy;
-            dB[0] += fb[0] * yz; dB[1] += fb[1] * xz; dB[2] += fb[2] * xy;
-            dC[0] += fc[0] * yz; dC[1] += fc[1] * xz; dC[2] += fc[2] * xy;
-          }
-        }
-      }
-    }
-    // block reduction of the nine partials; thread 0 adds to the four centres
-    double part[9] = {double(dA[0]), double(dA[1]), double(dA[2]), double(dB[0]), double(dB[1]),
-                      double(dB[2]), double(dC[0]), double(dC[1]), double(dC[2])};
-#pragma unroll
-    for (int q = 0; q < 9; ++q) {
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) part[q] += __shfl_down_sync(0xffffffffu, part[q], off);
-      if (lane == 0) red[q][warp] = part[q];
-    }
-    __syncthreads();
-    if (tid == 0) {
-      double sum[9];
-#pragma unroll
-      for (int q = 0; q < 9; ++q) {
-        sum[q] = 0.0;
-        for (int wi = 0; wi < GB::THREADS / 32; ++wi) sum[q] += red[q][wi];
-      }
-      double* gA = args.grad + 3LL * args.ws_atm[g.A];
-      double* gB = args.grad + 3LL * args.ws_atm[g.B];
-      double* gC = args.grad + 3LL * args.ws_atm[g.C];
-      double* gD = args.grad + 3LL * args.ws_atm[g.D];
-#pragma unroll
-      for (int x = 0; x < 3; ++x) {
-        atomicAdd(gA + x, sum[x]);
-        atomicAdd(gB + x, sum[3 + x]);
-        atomicAdd(gC + x, sum[6 + x]);
-        atomicAdd(gD + x, -(sum[x] + sum[3 + x] + sum[6 + x]));
-      }
-    }
-    __syncthreads();   // red and gam are rewritten by the next quartet
-  }
-}
 
 // Register-path coordinate VJP for small classes: one lane per ket of a
 // work item (warp-granular items as the J/K register path), the raised 2D
@@ -336,7 +82,7 @@ struct GradReg {
 template <int LA, int LB, int LC, int LD, typename R>
 __global__ void __launch_bounds__(128, 3) grad_reg_kernel(JKArgs args) {
   using CI = ClassInfo<LA, LB, LC, LD>;
-  using GC = GradCfg<LA, LB, LC, LD, 1>;
+  using GC = GradCfg<LA, LB, LC, LD>;
   using GI = GIdx<LA + 1, LB + 1, LC + 1, LD>;
   constexpr int N = GC::NROOT;
   constexpr int NGR = GradReg<LA, LB, LC, LD>::NGR;
@@ -448,49 +194,6 @@ __global__ void __launch_bounds__(128, 3) grad_reg_kernel(JKArgs args) {
   }
 }
 
-// Warp-per-quartet coordinate VJP for the classes between the lane kernel
-// and the block kernel (up to 48 KB of tables per warp).  Per primitive
-// quartet the raised 2D tables of every (root, axis) are built in shared
-// memory (build_g_mem, recursion scratch in shared memory, so the kernel's
-// registers stay those of the accumulation), then turned into derivative
-// tables: for every unraised (a, b, c, d) tuple the four values
-// (G, 2 alpha G(a+1) - a G(a-1), 2 beta G(b+1) - b G(b-1),
-// 2 gamma G(c+1) - c G(c-1)) side by side, so an element's nine partials at
-// one root take six 16-byte shared loads.  Lanes stride over the elements;
-// Gamma is staged in shared memory once per quartet.
-template <int LA, int LB, int LC, int LD>
-struct GradWarp {
-  using CI = ClassInfo<LA, LB, LC, LD>;
-  using GC = GradCfg<LA, LB, LC, LD, 1>;
-  static constexpr int N = GC::NROOT, NGR = GC::NG;
-  static constexpr int NGU = CI::NG;                                     // unraised tuples
-  static constexpr int NW = (LA + LB + 3) * (LC + LD + 2) * (LD + 1);   // build_g_mem scratch
-  static constexpr int D_OFF = (3 * N * NGR + 3) / 4 * 4;                // 16-byte aligned in FP32 and FP64
-  // the derivative tables overwrite the recursion scratch (dead by then)
-  static constexpr int DW = 3 * N * NGU * 4 > 3 * N * NW ? 3 * N * NGU * 4 : 3 * N * NW;
-  static constexpr int GAM_OFF = D_OFF + DW;
-  static constexpr int R_OFF = GAM_OFF + CI::NOUT;
-  static constexpr int ELEMS = (R_OFF + 2 * N + 3) / 4 * 4;
-  static constexpr int WARPS = 4;
-  static constexpr int NK = (CI::NOUT + 31) / 32;
-  static constexpr size_t bytes() { return (size_t)WARPS * ELEMS * sizeof(double); }   // FP64; FP32 takes half
-  // the classes where it beat the team / block kernel, measured per class
-  // on (H2O)16 cc-pVTZ (one VJP, serial launches): (21|21) 1.39x, (31|30)
-  // 1.61x, (33|10) 1.42x, (30|30) 1.38x, (33|00) 1.30x, (31|20) 1.25x,
-  // (31|11) 1.22x, (33|20) 1.20x, (32|10) 1.18x, (22|20) 1.12x, (32|30)
-  // 1.08x, (22|11) 1.05x, (30|22) 1.04x, (31|21) 1.03x, (22|21) 1.02x;
-  // elsewhere it was slower (to 0.69x) and is not used
-  static constexpr bool PICK = (LA == 2 && LB == 1 && LC == 2 && LD == 1) || (LA == 3 && LB == 1 && LC == 3 && LD == 0) ||
-                               (LA == 3 && LB == 3 && LC == 1 && LD == 0) || (LA == 3 && LB == 0 && LC == 3 && LD == 0) ||
-                               (LA == 3 && LB == 3 && LC == 0 && LD == 0) || (LA == 3 && LB == 1 && LC == 2 && LD == 0) ||
-                               (LA == 3 && LB == 1 && LC == 1 && LD == 1) || (LA == 3 && LB == 3 && LC == 2 && LD == 0) ||
-                               (LA == 3 && LB == 2 && LC == 1 && LD == 0) || (LA == 2 && LB == 2 && LC == 2 && LD == 0) ||
-                               (LA == 3 && LB == 2 && LC == 3 && LD == 0) || (LA == 2 && LB == 2 && LC == 1 && LD == 1) ||
-                               (LA == 3 && LB == 0 && LC == 2 && LD == 2) || (LA == 3 && LB == 1 && LC == 2 && LD == 1) ||
-                               (LA == 2 && LB == 2 && LC == 2 && LD == 1);
-  static constexpr bool OK = PICK && NGU <= 256 && ELEMS * sizeof(double) <= 48 * 1024;
-};
-
 // Four derivative-table values (G, f_A, f_B, f_C) stored side by side: one
 // 16-byte access in FP32, two in FP64.
 template <typename R> struct Quad;
@@ -514,115 +217,243 @@ template <> struct Quad<float> {
   }
 };
 
-template <int LA, int LB, int LC, int LD, typename R>
-__global__ void __launch_bounds__(128) grad_warp_kernel(JKArgs args) {
-  using CI = ClassInfo<LA, LB, LC, LD>;
-  using GW = GradWarp<LA, LB, LC, LD>;
-  using GC = GradCfg<LA, LB, LC, LD, 1>;
-  constexpr int N = GW::N, NGR = GW::NGR, NGU = GW::NGU;
-  extern __shared__ __align__(16) unsigned char wsm_raw[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  R* G = reinterpret_cast<R*>(wsm_raw) + warp * GW::ELEMS;
-  R* D = G + GW::D_OFF;
-  R* scratch = D;
-  R* gam = G + GW::GAM_OFF;
-  R* roots = G + GW::R_OFF;
-  // the lane's elements: unraised tuple index per axis, 8 bits each
-  int tix[GW::NK];
+// ---------------------------------------------------------------------------
+// Raised 2D tables of one (root, axis) in memory, in two stages: the vertical
+// recursion (columns in registers) with the ket transfer, one thread per
+// table; then the bra transfer, independent for every ket pair (c, d), one
+// thread per (table, c, d).  RA, RB, RC are the raised shells; the table is
+// G[((a (RB+1) + b)(RC+1) + c)(LD+1) + d], `w` holds raised_scratch values.
+// ---------------------------------------------------------------------------
+template <int RA, int RB, int RC, int LD>
+__host__ __device__ constexpr int raised_scratch() { return (RA + RB + 1) * (RC + LD + 1) * (LD + 1); }
+
+template <int RA, int RB, int RC, int LD, typename R>
+__device__ __forceinline__ void raised_vertical(R c00, R c0p, R b10, R b01, R b00, R g00, R cd, R* w) {
+  constexpr int LAB = RA + RB, LCD = RC + LD;
+  auto W = [&](int e, int c, int d) -> R& { return w[(e * (LCD + 1) + c) * (LD + 1) + d]; };
+  R prev[LAB + 1], cur[LAB + 1];
+  cur[0] = g00;
+  cur[1] = c00 * g00;
 #pragma unroll
-  for (int q = 0; q < GW::NK; ++q) {
-    const int o = lane + 32 * q;
-    tix[q] = 0;
-    if (o < CI::NOUT) {
-      const int id = o % CI::ND, ic = (o / CI::ND) % CI::NC;
-      const int ib = (o / CI::NCD) % CI::NB, ia = o / (CI::NCD * CI::NB);
-      const int tx = GIdx<LA, LB, LC, LD>::idx(cart_lx(LA, ia), cart_lx(LB, ib), cart_lx(LC, ic), cart_lx(LD, id));
-      const int ty = GIdx<LA, LB, LC, LD>::idx(cart_ly(LA, ia), cart_ly(LB, ib), cart_ly(LC, ic), cart_ly(LD, id));
-      const int tz = GIdx<LA, LB, LC, LD>::idx(cart_lz(LA, ia), cart_lz(LB, ib), cart_lz(LC, ic), cart_lz(LD, id));
-      tix[q] = tx | (ty << 8) | (tz << 16);
+  for (int e = 1; e < LAB; ++e) cur[e + 1] = c00 * cur[e] + R(e) * b10 * cur[e - 1];
+#pragma unroll
+  for (int e = 0; e <= LAB; ++e) {
+    W(e, 0, 0) = cur[e];
+    prev[e] = R(0);
+  }
+#pragma unroll 1
+  for (int f = 0; f < LCD; ++f) {
+    R next[LAB + 1];
+    const R fb = R(f) * b01;
+#pragma unroll
+    for (int e = 0; e <= LAB; ++e) {
+      R val = c0p * cur[e] + fb * prev[e];
+      if (e > 0) val += R(e) * b00 * cur[e - 1];
+      next[e] = val;
+    }
+#pragma unroll
+    for (int e = 0; e <= LAB; ++e) {
+      prev[e] = cur[e];
+      cur[e] = next[e];
+      W(e, f + 1, 0) = next[e];
     }
   }
+  if constexpr (LD > 0) {
+#pragma unroll 1
+    for (int e = 0; e <= LAB; ++e)
+#pragma unroll
+      for (int d = 1; d <= LD; ++d)
+#pragma unroll
+        for (int c = 0; c <= LCD - d; ++c) W(e, c, d) = W(e, c + 1, d - 1) + cd * W(e, c, d - 1);
+  }
+}
+
+// `q` = c (LD+1) + d, c <= RC.
+template <int RA, int RB, int RC, int LD, typename R>
+__device__ __forceinline__ void raised_bra(R ab, const R* w, int q, R* G) {
+  constexpr int LAB = RA + RB, KET = (RC + LD + 1) * (LD + 1), ROW = (RC + 1) * (LD + 1);
+  R y[LAB + 1];
+#pragma unroll
+  for (int e = 0; e <= LAB; ++e) y[e] = w[e * KET + q];
+#pragma unroll
+  for (int b = 0; b <= RB; ++b) {
+#pragma unroll
+    for (int a = 0; a <= RA; ++a) G[(a * (RB + 1) + b) * ROW + q] = y[a];
+    if (b < RB) {
+#pragma unroll
+      for (int a = 0; a + b < LAB; ++a) y[a] = y[a + 1] + ab * y[a];
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Coordinate VJP of every class off the register and lane kernels: a team (a
+// warp, or the block of 128 threads for the large blocks) takes one quartet
+// and in it batches of RB (primitive quartet, root) units.  Per batch the team
+// builds the raised tables (raised_vertical, raised_bra), turns them into
+// (value, d/dA, d/dB, d/dC) per (unit, axis, unraised index tuple) -- four
+// values side by side, one or two 16-byte loads -- and sums the nine centre
+// partials over the (unit, element) pairs; Gamma stays in shared memory per
+// quartet.  What bounds these classes is latency (few quartets, long chains):
+// the forms this replaces built one primitive quartet's tables on 3 N threads
+// at a time and recomputed each element's derivative factors from the table.
+// (H2O)4 cc-pVTZ split VJP 42.2 -> 33.9 ms (serial class times 70 -> 40).
+// ---------------------------------------------------------------------------
+template <int LA, int LB, int LC, int LD, typename R>
+struct GradUnit {
+  using CI = ClassInfo<LA, LB, LC, LD>;
+  static constexpr int THREADS = 128;
+#ifndef B200JK_GRAD_TEAM_NOUT
+#define B200JK_GRAD_TEAM_NOUT 400
+#endif
+  static constexpr int TEAM = CI::NOUT <= B200JK_GRAD_TEAM_NOUT ? 32 : THREADS, TEAMS = THREADS / TEAM;
+  static constexpr int N = (CI::L + 1) / 2 + 1;
+  static constexpr int B1 = LB + 2, C1 = LC + 2, D1 = LD + 1;
+  static constexpr int NG = (((LA + 2) * B1 * C1 * D1) + 3) / 4 * 4;   // 16-byte multiples keep the quads aligned
+  static constexpr int NW = raised_scratch<LA + 1, LB + 1, LC + 1, LD>();
+  static constexpr int NGU = CI::NG;
+  static constexpr int SIDE = ((NW > 4 * NGU ? NW : 4 * NGU) + 3) / 4 * 4;   // scratch, then the quads
+  static constexpr int TS = NG + SIDE, UNIT = 3 * TS;
+  static constexpr int NEL = (CI::NOUT + 3) / 4 * 4;
+#ifndef B200JK_GRAD_UNIT_KB
+#define B200JK_GRAD_UNIT_KB 72
+#endif
+  static constexpr int FIT = (int)((B200JK_GRAD_UNIT_KB * 1024 / sizeof(R) / TEAMS - NEL) / UNIT);
+  static constexpr int CAP = TEAM == 32 ? 10 : 42;   // 3 tables per unit fill the team
+  static constexpr int RB =
+      (int)(B200JK_GRAD_UNIT_KB * 1024 / sizeof(R) / TEAMS) < NEL + UNIT ? 1 : (FIT > CAP ? CAP : FIT);
+  static constexpr int TEAM_ELEMS = NEL + RB * UNIT;
+  static constexpr size_t bytes() { return (size_t)TEAMS * TEAM_ELEMS * sizeof(R); }
+  static_assert(bytes() <= 220 * 1024, "gradient batch exceeds shared memory");
+};
+
+template <int LA, int LB, int LC, int LD, typename R>
+__global__ void __launch_bounds__(128) grad_unit_kernel(JKArgs args) {
+  using CI = ClassInfo<LA, LB, LC, LD>;
+  using GU = GradUnit<LA, LB, LC, LD, R>;
+  constexpr int TEAM = GU::TEAM, TEAMS = GU::TEAMS, N = GU::N, NGU = GU::NGU, RB = GU::RB, NO = CI::NOUT;
+  constexpr int GRP = NO >= TEAM ? 1 : (TEAM / NO < RB ? TEAM / NO : RB);   // threads sharing an element
+  constexpr int NCMP = CI::NA + CI::NB + CI::NC + CI::ND;
+  extern __shared__ __align__(16) unsigned char gu_raw[];
+  __shared__ R s_ex[TEAMS][RB][3];
+  __shared__ double red[9][4];
+  __shared__ int tup[3][NCMP];
+  const int team = threadIdx.x / TEAM, tid = threadIdx.x % TEAM;
+  R* gam = reinterpret_cast<R*>(gu_raw) + (size_t)team * GU::TEAM_ELEMS;
+  R* units = gam + GU::NEL;
+  R(*ex)[3] = s_ex[team];
+  auto sync = [] {
+    if constexpr (TEAM == 32) __syncwarp();
+    else __syncthreads();
+  };
+  // an element's unraised tuple along each axis is a sum over its four components
+  for (int t = threadIdx.x; t < NCMP; t += GU::THREADS) {
+    const int which = t < CI::NA ? 0 : t < CI::NA + CI::NB ? 1 : t < CI::NA + CI::NB + CI::NC ? 2 : 3;
+    const int c = t - (which > 0 ? CI::NA : 0) - (which > 1 ? CI::NB : 0) - (which > 2 ? CI::NC : 0);
+    const int l = which == 0 ? LA : which == 1 ? LB : which == 2 ? LC : LD;
+    const int stride = which == 0 ? (LB + 1) * (LC + 1) * (LD + 1)
+                                  : which == 1 ? (LC + 1) * (LD + 1) : which == 2 ? (LD + 1) : 1;
+    tup[0][t] = cart_lx(l, c) * stride;
+    tup[1][t] = cart_ly(l, c) * stride;
+    tup[2][t] = cart_lz(l, c) * stride;
+  }
+  __syncthreads();
   const int4 w = args.work[blockIdx.x];
   const int bra = args.bra_pairs[w.x];
   int kb, ke;
   grad_ket_range(args, blockIdx.x, w, kb, ke);
-  for (int k = kb + warp; k < ke; k += GW::WARPS) {
+  for (int k = kb + team; k < ke; k += TEAMS) {
     QuartetGeom g;
     load_quartet(args, bra, args.ket_pairs[k], g);
     const long long base = args.mol_base[g.mol];
     const int n = args.mol_n[g.mol];
-    for (int o = lane; o < CI::NOUT; o += 32) {
-      const int id = o % CI::ND, ic = (o / CI::ND) % CI::NC;
-      const int ib = (o / CI::NCD) % CI::NB, ia = o / (CI::NCD * CI::NB);
+    for (int o = tid; o < NO; o += TEAM) {
+      const int id = o % CI::ND, ic = (o / CI::ND) % CI::NC, ib = (o / CI::NCD) % CI::NB, ia = o / (CI::NCD * CI::NB);
       gam[o] = R(g.scale * gamma_abcd(args, base, n, g.aoA + ia, g.aoB + ib, g.aoC + ic, g.aoD + id));
     }
     R dA[3] = {0, 0, 0}, dB[3] = {0, 0, 0}, dC[3] = {0, 0, 0};
-    for (int i = g.ppa; i < g.ppa + g.npa; ++i) {
-      const R alpha = R(args.pp_exp[i].x), beta = R(args.pp_exp[i].y);
-      for (int j = g.ppc; j < g.ppc + g.npc; ++j) {
+    const int nunit = g.npa * g.npc * N;
+    for (int u0 = 0; u0 < nunit; u0 += RB) {
+      const int nu = min(RB, nunit - u0);
+      sync();   // the previous batch's quads are no longer read
+      for (int t = tid; t < 3 * nu; t += TEAM) {
+        const int u = t / 3, ax = t - 3 * u;
+        const int p = (u0 + u) / N, r = (u0 + u) - p * N;
+        const int i = g.ppa + p / g.npc, j = g.ppc + p % g.npc;
         PrimQ<R> s;
         grad_prim<R>(args, g, i, j, s);
-        const R gamma_c = R(args.pp_exp[j].x);
-        __syncwarp();   // the previous primitive quartet's tables are no longer read
-        if (lane < 2 * N) roots[lane] = rys_one<N, R>(s.t, lane, args.tb);
-        __syncwarp();
-        if (lane < 3 * N) {
-          const int r = lane / 3, ax = lane - 3 * r;
-          RootCoef<R> rc;
-          root_coef<R>(s, roots[r], rc);
-          const R abd = R(ax == 0 ? g.abx : (ax == 1 ? g.aby : g.abz));
-          const R cdd = R(ax == 0 ? g.cdx : (ax == 1 ? g.cdy : g.cdz));
-          const R g00 = ax == 2 ? roots[N + r] * s.pref : R(1);
-          build_g_mem<LA + 1, LB + 1, LC + 1, LD, R>(rc.c00[ax], rc.c0p[ax], rc.b10, rc.b01, rc.b00, g00, abd, cdd,
-                                                    G + lane * NGR, scratch + lane * GW::NW);
-        }
-        __syncwarp();
-        const R e2a = R(2) * alpha, e2b = R(2) * beta, e2c = R(2) * gamma_c;
-        for (int e = lane; e < 3 * N * NGU; e += 32) {
-          const int tbl = e / NGU, tt = e - tbl * NGU;
-          const int d = tt % (LD + 1), c = (tt / (LD + 1)) % (LC + 1);
-          const int b = (tt / ((LD + 1) * (LC + 1))) % (LB + 1), a = tt / ((LD + 1) * (LC + 1) * (LB + 1));
-          const R* Gt = G + tbl * NGR;
-          const R v = Gt[GC::idx(a, b, c, d)];
-          R fa = e2a * Gt[GC::idx(a + 1, b, c, d)];
-          R fb = e2b * Gt[GC::idx(a, b + 1, c, d)];
-          R fc = e2c * Gt[GC::idx(a, b, c + 1, d)];
-          if (a) fa -= R(a) * Gt[GC::idx(a - 1, b, c, d)];
-          if (b) fb -= R(b) * Gt[GC::idx(a, b - 1, c, d)];
-          if (c) fc -= R(c) * Gt[GC::idx(a, b, c - 1, d)];
-          Quad<R>::st(D + 4 * e, v, fa, fb, fc);
-        }
-        __syncwarp();
+        RootCoef<R> rc;
+        root_coef<R>(s, rys_one<N, R>(s.t, r, args.tb), rc);
+        const R cdd = R(ax == 0 ? g.cdx : (ax == 1 ? g.cdy : g.cdz));
+        const R c00 = ax == 0 ? rc.c00[0] : (ax == 1 ? rc.c00[1] : rc.c00[2]);
+        const R c0p = ax == 0 ? rc.c0p[0] : (ax == 1 ? rc.c0p[1] : rc.c0p[2]);
+        const R g00 = ax == 2 ? rys_one<N, R>(s.t, N + r, args.tb) * s.pref : R(1);
+        raised_vertical<LA + 1, LB + 1, LC + 1, LD, R>(c00, c0p, rc.b10, rc.b01, rc.b00, g00, cdd,
+                                                       units + t * GU::TS + GU::NG);
+        ex[u][ax] = R(2) * R(ax == 0 ? args.pp_exp[i].x : ax == 1 ? args.pp_exp[i].y : args.pp_exp[j].x);
+      }
+      sync();
+      for (int t = tid; t < 3 * nu * GU::C1 * GU::D1; t += TEAM) {
+        const int ua = t / (GU::C1 * GU::D1), q = t - ua * (GU::C1 * GU::D1), ax = ua % 3;
+        const R abd = R(ax == 0 ? g.abx : (ax == 1 ? g.aby : g.abz));
+        raised_bra<LA + 1, LB + 1, LC + 1, LD, R>(abd, units + ua * GU::TS + GU::NG, q, units + ua * GU::TS);
+      }
+      sync();
+      for (int t = tid; t < 3 * nu * NGU; t += TEAM) {
+        const int ua = t / NGU, q = t - ua * NGU, u = ua / 3;
+        const int d = q % (LD + 1), c = (q / (LD + 1)) % (LC + 1);
+        const int b = (q / ((LD + 1) * (LC + 1))) % (LB + 1), a = q / ((LD + 1) * (LC + 1) * (LB + 1));
+        const R* G = units + ua * GU::TS + ((a * GU::B1 + b) * GU::C1 + c) * GU::D1 + d;
+        R fa = ex[u][0] * G[GU::B1 * GU::C1 * GU::D1], fb = ex[u][1] * G[GU::C1 * GU::D1], fc = ex[u][2] * G[GU::D1];
+        if (a) fa -= R(a) * G[-GU::B1 * GU::C1 * GU::D1];
+        if (b) fb -= R(b) * G[-GU::C1 * GU::D1];
+        if (c) fc -= R(c) * G[-GU::D1];
+        Quad<R>::st(units + ua * GU::TS + GU::NG + 4 * q, G[0], fa, fb, fc);
+      }
+      sync();
+      for (int t = tid; t < GRP * NO; t += TEAM) {
+        const int grp = t / NO, o = t - grp * NO;
+        const R gq = gam[o];
+        if (gq == R(0)) continue;
+        const int id = o % CI::ND, ic = (o / CI::ND) % CI::NC, ib = (o / CI::NCD) % CI::NB, ia = o / (CI::NCD * CI::NB);
+        int tx[3];
 #pragma unroll
-        for (int q = 0; q < GW::NK; ++q) {
-          const int o = lane + 32 * q;
-          if (o >= CI::NOUT) break;
-          const R gq = gam[o];
-          if (gq == R(0)) continue;
-          const int tx = tix[q] & 255, ty = (tix[q] >> 8) & 255, tz = tix[q] >> 16;
+        for (int x = 0; x < 3; ++x)
+          tx[x] = GU::NG + x * GU::TS +
+                  4 * (tup[x][ia] + tup[x][CI::NA + ib] + tup[x][CI::NA + CI::NB + ic] +
+                       tup[x][CI::NA + CI::NB + CI::NC + id]);
 #pragma unroll 2
-          for (int r = 0; r < N; ++r) {
-            const R* Dr = D + 4 * (3 * r * NGU);
-            R vx, ax, bx, cx, vy, ay, by, cy, vz, az, bz, cz;
-            Quad<R>::ld(Dr + 4 * tx, vx, ax, bx, cx);
-            Quad<R>::ld(Dr + 4 * (NGU + ty), vy, ay, by, cy);
-            Quad<R>::ld(Dr + 4 * (2 * NGU + tz), vz, az, bz, cz);
-            const R yz = gq * vy * vz, xz = gq * vx * vz, xy = gq * vx * vy;
-            dA[0] += ax * yz; dA[1] += ay * xz; dA[2] += az * xy;
-            dB[0] += bx * yz; dB[1] += by * xz; dB[2] += bz * xy;
-            dC[0] += cx * yz; dC[1] += cy * xz; dC[2] += cz * xy;
-          }
+        for (int u = grp; u < nu; u += GRP) {
+          const R* U = units + u * GU::UNIT;
+          R vx, ax, bx, cx, vy, ay, by, cy, vz, az, bz, cz;
+          Quad<R>::ld(U + tx[0], vx, ax, bx, cx);
+          Quad<R>::ld(U + tx[1], vy, ay, by, cy);
+          Quad<R>::ld(U + tx[2], vz, az, bz, cz);
+          const R yz = gq * vy * vz, xz = gq * vx * vz, xy = gq * vx * vy;
+          dA[0] += ax * yz; dA[1] += ay * xz; dA[2] += az * xy;
+          dB[0] += bx * yz; dB[1] += by * xz; dB[2] += bz * xy;
+          dC[0] += cx * yz; dC[1] += cy * xz; dC[2] += cz * xy;
         }
       }
     }
-    // warp reduction of the nine partials; lane 0 adds to the four centres
     double part[9] = {double(dA[0]), double(dA[1]), double(dA[2]), double(dB[0]), double(dB[1]),
                       double(dB[2]), double(dC[0]), double(dC[1]), double(dC[2])};
 #pragma unroll
-    for (int x = 0; x < 9; ++x)
+    for (int q = 0; q < 9; ++q)
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1) part[x] += __shfl_down_sync(0xffffffffu, part[x], off);
-    if (lane == 0) {
+      for (int off = 16; off > 0; off >>= 1) part[q] += __shfl_down_sync(0xffffffffu, part[q], off);
+    if constexpr (TEAM != 32) {
+      if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+        for (int q = 0; q < 9; ++q) red[q][threadIdx.x >> 5] = part[q];
+      }
+      __syncthreads();
+      if (tid == 0) {
+#pragma unroll
+        for (int q = 0; q < 9; ++q) part[q] = red[q][0] + red[q][1] + red[q][2] + red[q][3];
+      }
+    }
+    if (tid == 0) {
       double* gA = args.grad + 3LL * args.ws_atm[g.A];
       double* gB = args.grad + 3LL * args.ws_atm[g.B];
       double* gC = args.grad + 3LL * args.ws_atm[g.C];
@@ -635,7 +466,7 @@ __global__ void __launch_bounds__(128) grad_warp_kernel(JKArgs args) {
         atomicAdd(gD + x, -(part[x] + part[3 + x] + part[6 + x]));
       }
     }
-    __syncwarp();   // Gamma is rewritten by the next quartet
+    sync();   // Gamma (and red) are rewritten by the next quartet
   }
 }
 
@@ -719,7 +550,7 @@ __device__ __forceinline__ void grad_lane_centre(const RootCoef<R>& rc, R g00, c
 template <int LA, int LB, int LC, int LD, typename R>
 __global__ void __launch_bounds__(128) grad_lane_kernel(JKArgs args) {
   using CI = ClassInfo<LA, LB, LC, LD>;
-  using GC = GradCfg<LA, LB, LC, LD, 1>;
+  using GC = GradCfg<LA, LB, LC, LD>;
   using GL = GradLane<LA, LB, LC, LD>;
   constexpr int N = GC::NROOT;
   extern __shared__ __align__(16) unsigned char s_gam_raw[];   // [NOUT][THREADS]

@@ -189,43 +189,12 @@ int launch_grad(const JKArgs& args, cudaStream_t stream) {
     grad_reg_kernel<LA, LB, LC, LD, R><<<(args.nwork + 3) / 4, 128, 0, stream>>>(args);
     return (int)cudaGetLastError();
   }
-#ifndef B200JK_GRAD_WARP
-#define B200JK_GRAD_WARP 1
-#endif
-  if constexpr (B200JK_GRAD_WARP && GradWarp<LA, LB, LC, LD>::OK) {
-    // the classes between: one warp per quartet, derivative tables in shared memory
-    using GW = GradWarp<LA, LB, LC, LD>;
-    constexpr size_t smem = GW::bytes() / 8 * RS;
-    static std::atomic<uint64_t> smem_done{0};
-    const cudaError_t ea = smem_opt_in(grad_warp_kernel<LA, LB, LC, LD, R>, smem, smem_done);
-    if (ea != cudaSuccess) return (int)ea;
-    grad_warp_kernel<LA, LB, LC, LD, R><<<args.nwork, 32 * GW::WARPS, smem, stream>>>(args);
-    return (int)cudaGetLastError();
-  }
-#ifndef B200JK_GRAD_BLOCK
-#define B200JK_GRAD_BLOCK 1
-#endif
-  if constexpr (B200JK_GRAD_BLOCK && GradBlk<LA, LB, LC, LD>::OK) {
-    // large classes: one quartet per block at a time (block-wide teams)
-    using GB = GradBlk<LA, LB, LC, LD>;
-    constexpr size_t smem = GB::bytes() / 8 * RS;
-    static std::atomic<uint64_t> smem_done{0};
-    const cudaError_t ea = smem_opt_in(grad_block_kernel<LA, LB, LC, LD, R>, smem, smem_done);
-    if (ea != cudaSuccess) return (int)ea;
-    grad_block_kernel<LA, LB, LC, LD, R><<<args.nwork, GB::THREADS, smem, stream>>>(args);
-    return (int)cudaGetLastError();
-  }
-  using CI = ClassInfo<LA, LB, LC, LD>;
-  constexpr int TEAM = CI::NOUT <= 8 ? 4 : CI::NOUT <= 64 ? 8 : CI::NOUT <= 256 ? 16 : 32;
-  using GC = GradCfg<LA, LB, LC, LD, TEAM>;
-  constexpr size_t per_team = GC::bytes() / 8 * RS;
-  int teams = 128 / TEAM;
-  while (teams > 1 && per_team * teams > 200 * 1024) --teams;
-  const size_t smem = per_team * teams;
+  using GU = GradUnit<LA, LB, LC, LD, R>;
+  constexpr size_t smem = GU::bytes();
   static std::atomic<uint64_t> smem_done{0};
-  const cudaError_t ea = smem_opt_in(grad_team_kernel<LA, LB, LC, LD, TEAM, R>, smem, smem_done);
+  const cudaError_t ea = smem_opt_in(grad_unit_kernel<LA, LB, LC, LD, R>, smem, smem_done);
   if (ea != cudaSuccess) return (int)ea;
-  grad_team_kernel<LA, LB, LC, LD, TEAM, R><<<args.nwork, teams * TEAM, smem, stream>>>(args);
+  grad_unit_kernel<LA, LB, LC, LD, R><<<args.nwork, GU::THREADS, smem, stream>>>(args);
   return (int)cudaGetLastError();
 }
 
