@@ -41,8 +41,6 @@ struct DispatchTable {
   JKLauncher flat64[kQuartetClasses][9] = {};
   bool grouped[kQuartetClasses] = {};    // the class pair takes grouped lists
   bool reg_path[kQuartetClasses] = {};   // either precision runs the register path
-  bool tile[kQuartetClasses] = {};       // the FP64 kernel is the tile path
-  int team[kQuartetClasses] = {};
 };
 
 inline int pair_class(int la, int lb) { return la * (la + 1) / 2 + lb; }   // la >= lb

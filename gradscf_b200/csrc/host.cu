@@ -899,7 +899,6 @@ static void fill_items(Plan& p, ClassPairWork& W, int force) {
   W.grouped_x = disp.grouped[cls] && !p.grouped[x].q.empty();
   W.grouped_y = disp.grouped[cls] && !p.grouped[y].q.empty();
   const bool grouped = W.grouped_x || W.grouped_y;
-  const int chunk0 = disp.reg_path[cls] ? B200JK_REG_CHUNK : std::max(8, 4 * (128 / disp.team[cls]));
   std::vector<int4> items;
   W.quartets = W.prim_quartets = 0;
   W.item_cost.clear();
@@ -915,12 +914,11 @@ static void fill_items(Plan& p, ClassPairWork& W, int force) {
   for (const int4& r : runs) {
     const int bp = r.x, lo = r.y, hi = r.z;
     const long long npa = X.npp_pos[bp], wq = npa * Y.npp_pos[lo];
-    int chunk = chunk0;
+    int chunk = B200JK_TILE_CHUNK;
     if (disp.reg_path[cls]) {
       chunk = shrink_kets((force > 0 && !grouped) ? force : reg_chunk(npa, Y.npp_pos[lo]), wq, budget);
     } else {
-      // blocks of several quartets (tile, team) or of one (grad_block_kernel)
-      if (disp.tile[cls] && B200JK_TILE_CHUNK > 0) chunk = B200JK_TILE_CHUNK;
+      // blocks of one or several quartets at a time (tile path, grad_unit_kernel)
       while (chunk > 1 && chunk * wq > block_budget) chunk /= 2;
     }
     for (int s = lo; s < hi; s += chunk) {

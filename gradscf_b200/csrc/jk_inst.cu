@@ -32,16 +32,6 @@ struct Policy {
   // run 3-6x faster there than on the tile path)
   static constexpr int LIMIT = sizeof(R) == 4 ? B200JK_REG_LIMIT32 : 96;
   static constexpr bool REG = (3 * CI::NG + CI::NOUT <= LIMIT) && CI::NROOT <= 3;
-  // tile path: kets up to d x d (NCD <= 36), bra pair fits one block; FP32
-  // accumulators take half the registers, so FP32 takes kets up to f x s / d x p
-#ifndef B200JK_TILE_NCD32
-#define B200JK_TILE_NCD32 100   // measured on (H2O)8 cc-pVTZ: split kernels 92.5 -> 84.8 ms
-#endif
-#ifndef B200JK_TILE_NCD64
-#define B200JK_TILE_NCD64 100  // measured on (H2O)8 cc-pVTZ: FP64 kernels 102.0 -> 91.4 ms (despite spills)
-#endif
-  static constexpr int TILE_NCD = sizeof(R) == 4 ? B200JK_TILE_NCD32 : B200JK_TILE_NCD64;
-  static constexpr bool TILE = !REG && CI::NCD <= TILE_NCD && CI::NAB <= 128;
   static constexpr int TEAM = CI::NOUT <= 4 * 24 ? 4 : CI::NOUT <= 8 * 24 ? 8 : CI::NOUT <= 16 * 24 ? 16 : 32;
 };
 
@@ -51,22 +41,12 @@ int launch_class(const JKArgs& args, cudaStream_t stream) {
   using P = Policy<LA, LB, LC, LD, R>;
   if constexpr (P::REG) {
     jk_reg_kernel<LA, LB, LC, LD, R><<<(args.nwork + kRegWarps - 1) / kRegWarps, 32 * kRegWarps, 0, stream>>>(args);
-  } else if constexpr (P::TILE) {
-    using TC = TileCfg<LA, LB, LC, LD, R>;
-    constexpr size_t smem = TC::bytes();
-    static std::atomic<uint64_t> smem_done{0};
-    smem_opt_in(jk_tile_kernel<LA, LB, LC, LD, R>, smem, smem_done);
-    jk_tile_kernel<LA, LB, LC, LD, R><<<args.nwork, TC::THREADS, smem, stream>>>(args);
   } else {
-    constexpr int TEAM = P::TEAM;
-    using SM = TeamSmem<LA, LB, LC, LD, R, TEAM>;
-    constexpr size_t per_team = SM::bytes();
-    int teams = 128 / TEAM;
-    while (teams > 1 && per_team * teams > 200 * 1024) --teams;
-    const size_t smem = per_team * teams;
+    constexpr size_t smem = TileCfg<LA, LB, LC, LD, R>::bytes();
     static std::atomic<uint64_t> smem_done{0};
-    smem_opt_in(jk_team_kernel<LA, LB, LC, LD, R, TEAM>, smem, smem_done);
-    jk_team_kernel<LA, LB, LC, LD, R, TEAM><<<args.nwork, teams * TEAM, smem, stream>>>(args);
+    const cudaError_t ea = smem_opt_in(jk_tile_kernel<LA, LB, LC, LD, R>, smem, smem_done);
+    if (ea != cudaSuccess) return (int)ea;
+    jk_tile_kernel<LA, LB, LC, LD, R><<<args.nwork, TileCfg<LA, LB, LC, LD, R>::THREADS, smem, stream>>>(args);
   }
   return (int)cudaGetLastError();
 }
@@ -276,7 +256,6 @@ void REG_NAME(BRA_CLASS, KET_CLASS)(DispatchTable& t) {
   t.geom[id] = &launch_geom<XA, XB, YA, YB>;
   t.store[id] = &launch_store<XA, XB, YA, YB>;
   t.reg_path[id] = Policy<XA, XB, YA, YB, float>::REG || Policy<XA, XB, YA, YB>::REG;
-  t.tile[id] = Policy<XA, XB, YA, YB>::TILE;
   t.grouped[id] = GROUPED;
   register_gen<1, 2>(t, id);
   register_gen<1, 4>(t, id);
@@ -286,9 +265,6 @@ void REG_NAME(BRA_CLASS, KET_CLASS)(DispatchTable& t) {
   register_gen<4, 1>(t, id);
   register_gen<4, 2>(t, id);
   register_gen<4, 4>(t, id);
-  t.team[id] = Policy<XA, XB, YA, YB>::REG ? 1
-               : (Policy<XA, XB, YA, YB>::TILE ? TileCfg<XA, XB, YA, YB, double>::THREADS / 4
-                                               : Policy<XA, XB, YA, YB>::TEAM);
 #if BRA_CLASS == KET_CLASS
   t.schwarz[X] = &launch_schwarz<XA, XB>;
 #endif

@@ -16,6 +16,8 @@
 // antisymmetric density part).  That is the reference's eight-permutation
 // scatter (csrc/direct_jk.cc:50-75) folded by the symmetry of D.
 #pragma once
+#include <cuda_pipeline.h>
+
 #include "common.cuh"
 #include "os_eri.cuh"
 
@@ -1849,70 +1851,6 @@ __device__ __forceinline__ void team_block(const JKArgs& args, const QuartetGeom
   }
 }
 
-template <int LA, int LB, int LC, int LD, int TEAM>
-__device__ __forceinline__ void team_digest(const JKArgs& args, const QuartetGeom& g,
-                                            const double* V, int lane) {
-  using CI = ClassInfo<LA, LB, LC, LD>;
-  constexpr int NA = CI::NA, NB = CI::NB, NC = CI::NC, ND = CI::ND;
-  constexpr int T0 = NA * NB, T1 = T0 + NC * ND, T2 = T1 + NA * NC, T3 = T2 + NA * ND,
-                T4 = T3 + NB * NC, T5 = T4 + NB * ND;
-  const double s = g.scale;
-  const long long base = args.mol_base[g.mol];
-  const int n = args.mol_n[g.mol];
-  for (int e = 0; e < args.ndm; ++e) {
-    const double* dm = args.dens + e * args.dstride + base;
-    const bool doj = args.with_j && e < args.nsym;
-    double* vj = doj ? args.vj + e * args.dstride + base : nullptr;
-    double* vk = args.vk + e * args.dstride + base;
-    for (int t = lane; t < T5; t += TEAM) {
-      double acc = 0.0;
-      if (t < T1) {
-        if (!doj) continue;
-        if (t < T0) {
-          const int a = t / NB, b = t % NB;
-          for (int c = 0; c < NC; ++c)
-            for (int d = 0; d < ND; ++d)
-              acc += V[((a * NB + b) * NC + c) * ND + d] * dm[(long long)(g.aoC + c) * n + g.aoD + d];
-          atomicAdd(vj + (long long)(g.aoA + a) * n + g.aoB + b, 2.0 * s * acc);
-        } else {
-          const int c = (t - T0) / ND, d = (t - T0) % ND;
-          for (int a = 0; a < NA; ++a)
-            for (int b = 0; b < NB; ++b)
-              acc += V[((a * NB + b) * NC + c) * ND + d] * dm[(long long)(g.aoA + a) * n + g.aoB + b];
-          atomicAdd(vj + (long long)(g.aoC + c) * n + g.aoD + d, 2.0 * s * acc);
-        }
-        continue;
-      }
-      if (!args.with_k) continue;
-      if (t < T2) {
-        const int a = (t - T1) / NC, c = (t - T1) % NC;
-        for (int b = 0; b < NB; ++b)
-          for (int d = 0; d < ND; ++d)
-            acc += V[((a * NB + b) * NC + c) * ND + d] * dm[(long long)(g.aoB + b) * n + g.aoD + d];
-        atomicAdd(vk + (long long)(g.aoA + a) * n + g.aoC + c, s * acc);
-      } else if (t < T3) {
-        const int a = (t - T2) / ND, d = (t - T2) % ND;
-        for (int b = 0; b < NB; ++b)
-          for (int c = 0; c < NC; ++c)
-            acc += V[((a * NB + b) * NC + c) * ND + d] * dm[(long long)(g.aoB + b) * n + g.aoC + c];
-        atomicAdd(vk + (long long)(g.aoA + a) * n + g.aoD + d, s * acc);
-      } else if (t < T4) {
-        const int b = (t - T3) / NC, c = (t - T3) % NC;
-        for (int a = 0; a < NA; ++a)
-          for (int d = 0; d < ND; ++d)
-            acc += V[((a * NB + b) * NC + c) * ND + d] * dm[(long long)(g.aoA + a) * n + g.aoD + d];
-        atomicAdd(vk + (long long)(g.aoB + b) * n + g.aoC + c, s * acc);
-      } else {
-        const int b = (t - T4) / ND, d = (t - T4) % ND;
-        for (int a = 0; a < NA; ++a)
-          for (int c = 0; c < NC; ++c)
-            acc += V[((a * NB + b) * NC + c) * ND + d] * dm[(long long)(g.aoA + a) * n + g.aoC + c];
-        atomicAdd(vk + (long long)(g.aoB + b) * n + g.aoD + d, s * acc);
-      }
-    }
-  }
-}
-
 template <int LA, int LB, int LC, int LD, typename R, int TEAM>
 struct TeamSmem {
   using TC = TeamCfg<LA, LB, LC, LD, TEAM>;
@@ -1930,127 +1868,367 @@ struct TeamSmem {
   }
 };
 
-template <int LA, int LB, int LC, int LD, typename R, int TEAM>
-__global__ void jk_team_kernel(JKArgs args) {
-  using SM = TeamSmem<LA, LB, LC, LD, R, TEAM>;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int lane = threadIdx.x % TEAM;
-  const int team = threadIdx.x / TEAM;
-  const int nteams = blockDim.x / TEAM;
-  const unsigned mask =
-      TEAM == 32 ? 0xffffffffu : (((1u << TEAM) - 1u) << ((threadIdx.x % 32) / TEAM * TEAM));
-  unsigned char* mine = smem_raw + (size_t)team * SM::bytes();
-  R* sm = reinterpret_cast<R*>(mine);
-  double* vsm = reinterpret_cast<double*>(mine + SM::vofs());
-  const int4 w = args.work[blockIdx.x];
-  int kb, ke;
-  ket_range(args, w, kb, ke);
-  const BraRec br = load_bra(args, w.x);
-  for (int k = kb + team; k < ke; k += nteams) {
-    QuartetGeom g;
-    load_quartet_rec(args, br, k, g);
-    team_block<LA, LB, LC, LD, R, TEAM>(args, g, sm, vsm, lane, mask);
-    team_digest<LA, LB, LC, LD, TEAM>(args, g, vsm, lane);
-    __syncwarp(mask);
-  }
-}
-
 // ---------------------------------------------------------------------------
-// Tile path for mid-size classes (ket shells up to d): a team of NAB lanes
-// per quartet, lane (a, b) owning one bra Cartesian pair and every ket pair
-// (c, d) of the block, so each root costs it 3 (LC+1)(LD+1) shared reads for
-// NC*ND outputs.  Kets of a work item share their primitive count and the
-// bra is fixed, so all teams of a block run the primitive loop in lockstep
-// (block barriers, no divergence).  Digestion stages the contracted block in
-// shared memory and spreads the target elements over the team.
+// Tile path (every class off the register path): a team of NAB lanes per
+// quartet, lane (a, b) owning one bra Cartesian pair and every ket pair (c, d)
+// of the block in registers, Q quartets (kets of one item: equal primitive
+// counts) per block.  Blocks of more than 60 FP64 values per lane are cut by c
+// over S lanes.
+//
+// Per batch of PB primitive quartets of every quartet the block builds the 2D
+// tables in two parallel stages -- a thread per (primitive quartet, root, axis)
+// runs the vertical recursion row by row and the ket transfer, then a thread
+// per (table, ket column) the bra transfer in place -- and every lane takes its
+// rows of all of them.  Digestion works from the registers: the four exchange
+// contractions of a lane's block and J[a][b] need the lane's own values alone,
+// so what goes through shared memory is 2 (NC + ND) exchange partials and the
+// NCD products with D[a][b] per lane, summed over the team's lanes; J[a][b]
+// stays in a register over the item.
+//
+// What bounds it is shared-memory wavefronts: 3 KSTR reads feed 2 NCD
+// operations per root and lane.  The form it replaces built one primitive
+// quartet's tables on 3 N threads at a time and digested from a staged block
+// (six reads of every element, rows NCD apart on four banks): (H2O)11 cc-pVTZ
+// FP64 class times (21|20) 8.2 -> 5.5 ms, (22|10) 6.8 -> 3.8, (32|10) 4.8 -> 2.8,
+// its split build 83.4 -> 57.3 ms; (H2O)6 cc-pVTZ FP64 25.6 -> 20.2 ms.
 // ---------------------------------------------------------------------------
 template <int LA, int LB, int LC, int LD, typename R>
 struct TileCfg {
   using CI = ClassInfo<LA, LB, LC, LD>;
   static constexpr int TEAM = CI::NAB;
   static constexpr int Q = (128 / TEAM) > 0 ? (128 / TEAM) : 1;      // quartets per block
-  static constexpr int THREADS = Q * TEAM;
+  static constexpr int S = CI::NCD * sizeof(R) > 60 * 8 ? 2 : 1;     // lanes sharing a (a, b) row by c
+  static constexpr int COLS = Q * TEAM, THREADS = S * COLS;
   static constexpr int N = CI::NROOT;
-  static constexpr int NG = CI::NG;
   static constexpr int KSTR = (LC + 1) * (LD + 1);                     // ket part of a G row
-  // per quartet slot: G (3N*NG R), roots (2N R), staged block (NOUT double)
-  static constexpr size_t G_BYTES = ((size_t)(3 * N * NG + 2 * N) * sizeof(R) + 15) / 16 * 16;
-  static constexpr size_t SLOT = G_BYTES + (size_t)CI::NOUT * 8;
-  static constexpr size_t bytes() { return SLOT * Q; }
+  // tables of one primitive quartet; odd strides keep the lanes of a stage on
+  // different banks
+  static constexpr int NGS = CI::NG | 1, UNIT = (3 * N * NGS) | 1;
+  static constexpr int FIT = (int)(64 * 1024 / sizeof(R)) / (Q * UNIT);
+  static constexpr int FILL = (THREADS + 3 * N * Q - 1) / (3 * N * Q);
+  static constexpr int PB = FIT < 1 ? 1 : (FILL < FIT ? FILL : FIT);
+  static constexpr size_t UNIT_BYTES = ((size_t)PB * Q * UNIT * sizeof(R) + 15) / 16 * 16;
+  // staged rows (one value per (a, b) lane, COLS of them): exchange partials
+  // over d and c, then the J[c][d] products, JCH of them at a time
+  static constexpr int KROWS = 2 * CI::NC + 2 * S * CI::ND, RS = COLS | 1;
+  static constexpr int JPASS = (CI::NCD + 35) / 36, JCH = (CI::NCD + JPASS - 1) / JPASS;
+  static constexpr size_t STAGE_BYTES = ((size_t)(KROWS + JCH) * RS * 8 + 15) / 16 * 16;
+  // density elements of one quartet: D[c][d], D[b][d], D[b][c], D[a][d], D[a][c]
+  static constexpr int D1 = CI::NCD, D2 = D1 + CI::NB * CI::ND, D3 = D2 + CI::NB * CI::NC,
+                       D4 = D3 + CI::NA * CI::ND, DTOT = D4 + CI::NA * CI::NC;
+  // the tables are no longer read when a block is digested: both share memory
+  static constexpr size_t MAIN = UNIT_BYTES > STAGE_BYTES ? UNIT_BYTES : STAGE_BYTES;
+  static constexpr size_t bytes() { return MAIN + (size_t)Q * DTOT * 8; }
 };
 
+// 2D integrals of one (root, axis) without the bra transfer, rows e = 0..LA+LB
+// of w[c (LD+1) + d], c <= LC: row e needs row e - 1 alone, so two rows are live.
 template <int LA, int LB, int LC, int LD, typename R>
-__global__ void __launch_bounds__(128) jk_tile_kernel(JKArgs args) {
+__device__ __forceinline__ void tile_rows(R c00, R c0p, R b10, R b01, R b00, R g00, R cd, R* w) {
+  constexpr int LAB = LA + LB, LCD = LC + LD, KSTR = (LC + 1) * (LD + 1);
+  R prev[LCD + 1], cur[LCD + 1];
+#pragma unroll
+  for (int e = 0; e <= LAB; ++e) {
+    R next[LCD + 1];
+    next[0] = e == 0 ? g00 : c00 * cur[0];
+    if (e > 1) next[0] += R(e - 1) * b10 * prev[0];
+#pragma unroll
+    for (int f = 0; f < LCD; ++f) {
+      next[f + 1] = c0p * next[f];
+      if (f > 0) next[f + 1] += R(f) * b01 * next[f - 1];
+      if (e > 0) next[f + 1] += R(e) * b00 * cur[f];
+    }
+#pragma unroll
+    for (int f = 0; f <= LCD; ++f) {
+      prev[f] = cur[f];
+      cur[f] = next[f];
+    }
+#pragma unroll
+    for (int d = 0; d <= LD; ++d) {
+#pragma unroll
+      for (int c = 0; c <= LC; ++c) w[e * KSTR + c * (LD + 1) + d] = next[c];
+#pragma unroll
+      for (int c = 0; c < LCD - d; ++c) next[c] = next[c + 1] + cd * next[c];
+    }
+  }
+}
+
+// The bra transfer of one ket column, in place: G[(a (LB+1) + b) KSTR] from
+// the rows e KSTR (a column is read whole before it is written).
+template <int LA, int LB, int KSTR, typename R>
+__device__ __forceinline__ void tile_bra(R ab, R* G) {
+  constexpr int LAB = LA + LB;
+  R y[LAB + 1];
+#pragma unroll
+  for (int e = 0; e <= LAB; ++e) y[e] = G[e * KSTR];
+#pragma unroll
+  for (int b = 0; b <= LB; ++b) {
+#pragma unroll
+    for (int a = 0; a <= LA; ++a) G[(a * (LB + 1) + b) * KSTR] = y[a];
+    if (b < LB) {
+#pragma unroll
+      for (int a = 0; a + b < LAB; ++a) y[a] = y[a + 1] + ab * y[a];
+    }
+  }
+}
+
+// Geometry of the kets of the block's current quartets.
+struct TileKet {
+  double c[3], cd[3];
+  int ppc, aoC, aoD;
+  double scale;   // 0: no quartet here
+};
+
+// One lane's share of the element sums: rows c in [C0, C1).
+template <int LA, int LB, int LC, int LD, typename R, int C0, int C1>
+__device__ __forceinline__ void tile_elements(const R* units, int np, int bx, int by, int bz, R* acc) {
+  using CI = ClassInfo<LA, LB, LC, LD>;
+  using TC = TileCfg<LA, LB, LC, LD, R>;
+  for (int pp = 0; pp < np; ++pp) {
+    const R* U = units + (size_t)pp * TC::Q * TC::UNIT;
+#pragma unroll 1
+    for (int r = 0; r < TC::N; ++r, U += 3 * TC::NGS) {
+      const R *gx = U + bx, *gy = U + TC::NGS + by, *gz = U + 2 * TC::NGS + bz;
+      R vx[TC::KSTR], vy[TC::KSTR], vz[TC::KSTR];
+#pragma unroll
+      for (int q = 0; q < TC::KSTR; ++q) { vx[q] = gx[q]; vy[q] = gy[q]; vz[q] = gz[q]; }
+      static_for_n<(C1 - C0) * CI::ND>([&](auto O) {
+        constexpr int o = decltype(O)::value, ic = C0 + o / CI::ND, id = o % CI::ND;
+        constexpr int jx = cart_lx(LC, ic) * (LD + 1) + cart_lx(LD, id);
+        constexpr int jy = cart_ly(LC, ic) * (LD + 1) + cart_ly(LD, id);
+        constexpr int jz = cart_lz(LC, ic) * (LD + 1) + cart_lz(LD, id);
+        acc[o] += vx[jx] * vy[jy] * vz[jz];
+      });
+    }
+  }
+}
+
+// One lane's block against the density: exchange partials and J[c][d] products
+// to the stage (column `col`), the J[a][b] sum returned.
+template <int LA, int LB, int LC, int LD, typename R, int SL>
+__device__ __forceinline__ double tile_partials(const R* acc, const double* ds, double dab, int ia, int ib, int jpass,
+                                                bool doj, bool dok, double* stage) {
+  using CI = ClassInfo<LA, LB, LC, LD>;
+  using TC = TileCfg<LA, LB, LC, LD, R>;
+  constexpr int NC = CI::NC, ND = CI::ND, RS = TC::RS, C0 = SL * NC / TC::S, C1 = (SL + 1) * NC / TC::S;
+  double jab = 0.0;
+  if (jpass == 0) {
+    const double *bd = ds + TC::D1 + ib * ND, *bc = ds + TC::D2 + ib * NC;
+    const double *ad = ds + TC::D3 + ia * ND, *ac = ds + TC::D4 + ia * NC;
+    double dbd[ND], dad[ND], kad[ND], kbd[ND];
+#pragma unroll
+    for (int d = 0; d < ND; ++d) {
+      dbd[d] = bd[d];
+      dad[d] = ad[d];
+      kad[d] = kbd[d] = 0.0;
+    }
+    static_for_n<C1 - C0>([&](auto C) {
+      constexpr int o = decltype(C)::value, c = C0 + o;
+      const double dbc = bc[c], dac = ac[c];
+      double kac = 0.0, kbc = 0.0;
+      static_for_n<ND>([&](auto D) {
+        constexpr int d = decltype(D)::value;
+        const double v = double(acc[o * ND + d]);
+        jab += v * ds[c * ND + d];
+        kac += v * dbd[d];
+        kbc += v * dad[d];
+        kad[d] += v * dbc;
+        kbd[d] += v * dac;
+      });
+      if (dok) {
+        stage[c * RS] = kac;
+        stage[(NC + c) * RS] = kbc;
+      }
+    });
+    if (dok) {
+#pragma unroll
+      for (int d = 0; d < ND; ++d) {
+        stage[(2 * NC + SL * ND + d) * RS] = kad[d];
+        stage[(2 * NC + (TC::S + SL) * ND + d) * RS] = kbd[d];
+      }
+    }
+  }
+  if (doj) {
+    static_for_n<(C1 - C0) * ND>([&](auto O) {
+      constexpr int o = decltype(O)::value, cd = C0 * ND + o;
+      if (TC::JPASS == 1 || cd / TC::JCH == jpass)
+        stage[(TC::KROWS + cd % TC::JCH) * RS] = double(acc[o]) * dab;
+    });
+  }
+  return jab;
+}
+
+template <int LA, int LB, int LC, int LD, typename R>
+__global__ void __launch_bounds__(TileCfg<LA, LB, LC, LD, R>::THREADS) jk_tile_kernel(JKArgs args) {
   using CI = ClassInfo<LA, LB, LC, LD>;
   using TC = TileCfg<LA, LB, LC, LD, R>;
   using GI = GIdx<LA, LB, LC, LD>;
-  constexpr int N = TC::N, NG = TC::NG, TEAM = TC::TEAM;
+  constexpr int N = TC::N, NGS = TC::NGS, TEAM = TC::TEAM, Q = TC::Q, S = TC::S, RS = TC::RS;
+  constexpr int NA = CI::NA, NB = CI::NB, NC = CI::NC, ND = CI::ND;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ TileKet s_ket[Q];
   const int4 w = args.work[blockIdx.x];
   int kb, ke;
   ket_range(args, w, kb, ke);
   if (kb >= ke) return;
-  const int team = threadIdx.x / TEAM, lane = threadIdx.x % TEAM;
-  R* G = reinterpret_cast<R*>(smem_raw + (size_t)team * TC::SLOT);
-  R* roots = G + 3 * N * NG;
-  double* V = reinterpret_cast<double*>(smem_raw + (size_t)team * TC::SLOT + TC::G_BYTES);
+  R* units = reinterpret_cast<R*>(smem_raw);
+  double* stage = reinterpret_cast<double*>(smem_raw);
+  double* dens = reinterpret_cast<double*>(smem_raw + TC::MAIN);
+  // threads are slice-major, so a warp's lanes mostly run the same slice
+  const int slice = S == 1 ? 0 : threadIdx.x / TC::COLS, col = threadIdx.x - slice * TC::COLS;
+  const int team = col / TEAM, lane = col % TEAM;
   const BraRec br = load_bra(args, w.x);
+  const int npa = br.ix.y, npq = npa * args.ket_ix[kb].y;
+  QuartetGeom g;
+  g.ax = br.ra.x; g.ay = br.ra.y; g.az = br.ra.z;
+  g.omega2 = args.omega2;
+  const int mol = (int)br.ra.w, n = args.mol_n[mol];
+  const long long base = args.mol_base[mol];
   // this lane's bra Cartesian pair
-  const int ia = lane / CI::NB, ib = lane % CI::NB;
+  const int ia = lane / NB, ib = lane % NB;
   const int bx = GI::idx(cart_lx(LA, ia), cart_lx(LB, ib), 0, 0);
   const int by = GI::idx(cart_ly(LA, ia), cart_ly(LB, ib), 0, 0);
   const int bz = GI::idx(cart_lz(LA, ia), cart_lz(LB, ib), 0, 0);
-  for (int k0 = kb; k0 < ke; k0 += TC::Q) {
-    const bool active = k0 + team < ke;
-    QuartetGeom g;
-    load_quartet_rec(args, br, active ? k0 + team : ke - 1, g);
-    R acc[CI::NCD];
+  const long long ab = (long long)(br.ix.z + ia) * n + br.ix.w + ib;
+  double jab0 = 0.0;   // J[a][b] of the first density over the item
+  for (int k0 = kb; k0 < ke; k0 += Q) {
+    if (threadIdx.x < Q) {
+      const int k = min(k0 + (int)threadIdx.x, ke - 1);
+      QuartetGeom q;
+      load_quartet_rec(args, br, k, q);
+      s_ket[threadIdx.x] = TileKet{{q.cx, q.cy, q.cz}, {q.cdx, q.cdy, q.cdz}, q.ppc, q.aoC, q.aoD,
+                                   k0 + (int)threadIdx.x < ke ? q.scale : 0.0};
+    }
+    __syncthreads();
+    const TileKet& kt = s_ket[team];
+    auto fetch = [&](int e) {
+      const double* dm = args.dens + e * args.dstride + base;
+      double* ds = dens + team * TC::DTOT;
+      for (int t = slice * TEAM + lane; t < TC::DTOT; t += S * TEAM) {
+        int row, c;
+        if (t < TC::D1) { row = kt.aoC + t / ND; c = kt.aoD + t % ND; }
+        else if (t < TC::D2) { row = br.ix.w + (t - TC::D1) / ND; c = kt.aoD + (t - TC::D1) % ND; }
+        else if (t < TC::D3) { row = br.ix.w + (t - TC::D2) / NC; c = kt.aoC + (t - TC::D2) % NC; }
+        else if (t < TC::D4) { row = br.ix.z + (t - TC::D3) / ND; c = kt.aoD + (t - TC::D3) % ND; }
+        else { row = br.ix.z + (t - TC::D4) / NC; c = kt.aoC + (t - TC::D4) % NC; }
+        __pipeline_memcpy_async(ds + t, dm + (long long)row * n + c, 8);
+      }
+      __pipeline_commit();
+    };
+    fetch(0);   // arrives while the primitive quartets are evaluated
+    constexpr int ROWS = NC / S * ND;
+    static_assert(NC % S == 0, "slices of whole c rows");
+    R acc[ROWS];
 #pragma unroll
-    for (int q = 0; q < CI::NCD; ++q) acc[q] = R(0);
-    for (int j = g.ppc; j < g.ppc + g.npc; ++j) {
-      const double4 Qd = args.pp_data[j];
-      const double2 QA = args.pp_aux[j];
-      for (int i = g.ppa; i < g.ppa + g.npa; ++i) {
+    for (int q = 0; q < ROWS; ++q) acc[q] = R(0);
+    for (int p0 = 0; p0 < npq; p0 += TC::PB) {
+      const int np = min(TC::PB, npq - p0);
+      for (int t = threadIdx.x; t < np * Q * 3 * N; t += TC::THREADS) {
+        const int u = t / (3 * N), f = t - u * (3 * N), r = f / 3, ax = f - 3 * r;
+        const int slot = u % Q, p = p0 + u / Q, j = p / npa, i = p - j * npa;
+        const TileKet& kq = s_ket[slot];
+        QuartetGeom gq = g;
+        gq.cx = kq.c[0]; gq.cy = kq.c[1]; gq.cz = kq.c[2];
         PrimQ<R> s;
-        prim_setup<R>(g, args.pp_data[i], args.pp_aux[i], Qd, QA, s);
-        for (int f = lane; f < 2 * N; f += TEAM) roots[f] = rys_one<N, R>(s.t, f, args.tb);
-        __syncthreads();
-        for (int tsk = lane; tsk < 3 * N; tsk += TEAM) {
-          const int r = tsk / 3, ax = tsk - 3 * r;
-          RootCoef<R> rc;
-          root_coef<R>(s, roots[r], rc);
-          const R abd = ax == 0 ? R(g.abx) : (ax == 1 ? R(g.aby) : R(g.abz));
-          const R cdd = ax == 0 ? R(g.cdx) : (ax == 1 ? R(g.cdy) : R(g.cdz));
-          const R g00 = ax == 2 ? roots[N + r] * s.pref : R(1);
-          build_g<LA, LB, LC, LD, R>(rc.c00[ax], rc.c0p[ax], rc.b10, rc.b01, rc.b00, g00, abd, cdd,
-                                     G + (r * 3 + ax) * NG);
+        prim_setup<R>(gq, args.pp_data[br.ix.x + i], args.pp_aux[br.ix.x + i], args.pp_data[kq.ppc + j],
+                      args.pp_aux[kq.ppc + j], s);
+        RootCoef<R> rc;
+        root_coef<R>(s, rys_one<N, R>(s.t, r, args.tb), rc);
+        const R c00 = ax == 0 ? rc.c00[0] : (ax == 1 ? rc.c00[1] : rc.c00[2]);
+        const R c0p = ax == 0 ? rc.c0p[0] : (ax == 1 ? rc.c0p[1] : rc.c0p[2]);
+        const R g00 = ax == 2 ? rys_one<N, R>(s.t, N + r, args.tb) * s.pref : R(1);
+        tile_rows<LA, LB, LC, LD, R>(c00, c0p, rc.b10, rc.b01, rc.b00, g00, R(kq.cd[ax]),
+                                     units + (size_t)u * TC::UNIT + f * NGS);
+      }
+      __syncthreads();
+      if constexpr (LB > 0) {
+        for (int t = threadIdx.x; t < np * Q * 3 * N * TC::KSTR; t += TC::THREADS) {
+          const int tab = t / TC::KSTR, q = t - tab * TC::KSTR, u = tab / (3 * N), f = tab - u * (3 * N);
+          const R abd = R(f % 3 == 0 ? br.ab.x : (f % 3 == 1 ? br.ab.y : br.ab.z));
+          tile_bra<LA, LB, TC::KSTR, R>(abd, units + (size_t)u * TC::UNIT + f * NGS + q);
         }
         __syncthreads();
+      }
+      const R* mine = units + (size_t)team * TC::UNIT;
+      if (S == 1 || slice == 0) tile_elements<LA, LB, LC, LD, R, 0, NC / S>(mine, np, bx, by, bz, acc);
+      else if constexpr (S > 1) tile_elements<LA, LB, LC, LD, R, NC / S, NC>(mine, np, bx, by, bz, acc);
+      __syncthreads();
+    }
+    for (int e = 0; e < args.ndm; ++e) {
+      const double* dm = args.dens + e * args.dstride + base;
+      const bool doj = args.with_j && e < args.nsym;
+      double* vj = doj ? args.vj + e * args.dstride + base : nullptr;
+      double* vk = args.vk + e * args.dstride + base;
+      if (e > 0) fetch(e);
+      __pipeline_wait_prior(0);
+      __syncthreads();
+      const double* ds = dens + team * TC::DTOT;
+      const double dab = dm[ab], sc = kt.scale;
+      for (int jp = 0; jp < TC::JPASS; ++jp) {
+        if (jp > 0 && !doj) break;
+        double jab = 0.0;
+        if (S == 1 || slice == 0)
+          jab = tile_partials<LA, LB, LC, LD, R, 0>(acc, ds, dab, ia, ib, jp, doj, args.with_k, stage + col);
+        else if constexpr (S > 1)
+          jab = tile_partials<LA, LB, LC, LD, R, 1>(acc, ds, dab, ia, ib, jp, doj, args.with_k, stage + col);
+        if (e == 0) jab0 += 2.0 * sc * jab;
+        else if (doj && jp == 0 && sc != 0.0) atomicAdd(vj + ab, 2.0 * sc * jab);
+        __syncthreads();
+        // sums over the team's lanes: columns of the staged rows
+        constexpr int T0 = NA * NC, T1 = T0 + NA * ND, T2 = T1 + NB * NC, T3 = T2 + NB * ND;
+        const int njt = min(TC::JCH, CI::NCD - jp * TC::JCH);
+        const int first = jp == 0 && args.with_k ? 0 : T3, last = T3 + (doj ? njt : 0);
+        const double* st = stage + team * TEAM;
+        if (sc != 0.0) {
+          for (int t = first + slice * TEAM + lane; t < last; t += S * TEAM) {
+            double sum = 0.0;
+            if (t < T0) {
+              const int a = t / NC, c = t % NC;
 #pragma unroll
-        for (int r = 0; r < N; ++r) {
-          R vx[TC::KSTR], vy[TC::KSTR], vz[TC::KSTR];
-          const R* gx = G + (r * 3) * NG + bx;
-          const R* gy = G + (r * 3 + 1) * NG + by;
-          const R* gz = G + (r * 3 + 2) * NG + bz;
+              for (int b = 0; b < NB; ++b) sum += st[c * RS + a * NB + b];
+              atomicAdd(vk + (long long)(br.ix.z + a) * n + kt.aoC + c, sc * sum);
+            } else if (t < T1) {
+              const int a = (t - T0) / ND, d = (t - T0) % ND;
 #pragma unroll
-          for (int q = 0; q < TC::KSTR; ++q) { vx[q] = gx[q]; vy[q] = gy[q]; vz[q] = gz[q]; }
-          static_for<0, CI::NCD>([&](auto O) {
-            constexpr int cd = decltype(O)::value;
-            constexpr int ic = cd / CI::ND, id = cd % CI::ND;
-            constexpr int jx = cart_lx(LC, ic) * (LD + 1) + cart_lx(LD, id);
-            constexpr int jy = cart_ly(LC, ic) * (LD + 1) + cart_ly(LD, id);
-            constexpr int jz = cart_lz(LC, ic) * (LD + 1) + cart_lz(LD, id);
-            acc[cd] += vx[jx] * vy[jy] * vz[jz];
-          });
+              for (int x = 0; x < S; ++x)
+#pragma unroll
+                for (int b = 0; b < NB; ++b) sum += st[(2 * NC + x * ND + d) * RS + a * NB + b];
+              atomicAdd(vk + (long long)(br.ix.z + a) * n + kt.aoD + d, sc * sum);
+            } else if (t < T2) {
+              const int b = (t - T1) / NC, c = (t - T1) % NC;
+#pragma unroll
+              for (int a = 0; a < NA; ++a) sum += st[(NC + c) * RS + a * NB + b];
+              atomicAdd(vk + (long long)(br.ix.w + b) * n + kt.aoC + c, sc * sum);
+            } else if (t < T3) {
+              const int b = (t - T2) / ND, d = (t - T2) % ND;
+#pragma unroll
+              for (int x = 0; x < S; ++x)
+#pragma unroll
+                for (int a = 0; a < NA; ++a) sum += st[(2 * NC + (S + x) * ND + d) * RS + a * NB + b];
+              atomicAdd(vk + (long long)(br.ix.w + b) * n + kt.aoD + d, sc * sum);
+            } else {
+              const int cd = jp * TC::JCH + t - T3;
+              const double* row = st + (TC::KROWS + t - T3) * RS;
+#pragma unroll 4
+              for (int l = 0; l < TEAM; ++l) sum += row[l];
+              atomicAdd(vj + (long long)(kt.aoC + cd / ND) * n + kt.aoD + cd % ND, 2.0 * sc * sum);
+            }
+          }
         }
         __syncthreads();
       }
     }
+  }
+  if (args.with_j && args.nsym > 0) {
+    stage[slice * RS + col] = jab0;
+    __syncthreads();
+    if (threadIdx.x < TEAM) {
+      double sum = 0.0;
 #pragma unroll
-    for (int q = 0; q < CI::NCD; ++q) V[lane * CI::NCD + q] = double(acc[q]);
-    __syncthreads();
-    if (active) team_digest<LA, LB, LC, LD, TEAM>(args, g, V, lane);
-    __syncthreads();
+      for (int x = 0; x < S; ++x)
+        for (int q = 0; q < Q; ++q) sum += stage[x * RS + q * TEAM + lane];
+      atomicAdd(args.vj + base + ab, sum);
+    }
   }
 }
 
