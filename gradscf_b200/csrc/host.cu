@@ -1,7 +1,9 @@
 // Plan construction, basis transforms, J/K orchestration and the C ABI.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
+#include <exception>
 #include <map>
 #include <unordered_map>
 #include <set>
@@ -12,6 +14,8 @@
 #include <numeric>
 #include <stdexcept>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <tuple>
 #include <vector>
 
@@ -872,14 +876,17 @@ static void fill_group(GroupWork& G, const ClassList& X, const ClassList& Y, boo
     G.item_cost = std::move(cost);
   }
   G.nwork = (int)G.all_items.size();
-  CUDA_OK(G.work.ensure(std::max<size_t>(G.all_items.size(), 1) * sizeof(int4)));
-  if (!G.all_items.empty())
-    CUDA_OK(cudaMemcpy(G.work.ptr, G.all_items.data(), G.all_items.size() * sizeof(int4), cudaMemcpyHostToDevice));
-  CUDA_OK(G.m.ensure(std::max<size_t>(G.all_items.size(), 1) * sizeof(double)));
   // the FP64 flat list of split builds: room for 1/16 of the group's (bra,
   // ket) pairs, at most 2^21; items that do not fit keep the bra-group path
   const long long pairs = G.quartets / std::max(1, gb * gk);
   G.flat_cap = (int)std::min<long long>(pairs / 16 + 4096, 1LL << 21);
+}
+
+static void upload_group(GroupWork& G) {
+  CUDA_OK(G.work.ensure(std::max<size_t>(G.all_items.size(), 1) * sizeof(int4)));
+  if (!G.all_items.empty())
+    CUDA_OK(cudaMemcpy(G.work.ptr, G.all_items.data(), G.all_items.size() * sizeof(int4), cudaMemcpyHostToDevice));
+  CUDA_OK(G.m.ensure(std::max<size_t>(G.all_items.size(), 1) * sizeof(double)));
   CUDA_OK(G.flat.ensure((size_t)G.flat_cap * sizeof(int2)));
   CUDA_OK(G.flat_n.ensure(sizeof(unsigned long long)));
   CUDA_OK(G.skip.ensure(std::max<size_t>(G.all_items.size(), 1) * sizeof(int)));
@@ -888,8 +895,9 @@ static void fill_group(GroupWork& G, const ClassList& X, const ClassList& Y, boo
 // (Re)build the work items of class pair W: the expanded items and, where
 // both precisions' kernels take grouped lists, the grouped buckets.
 // `force` > 0 sets the ket chunk of the items the J/K build launches on the
-// register path (the autotuner's knob); 0 keeps the default rule.
-static void fill_items(Plan& p, ClassPairWork& W, int force) {
+// register path (the autotuner's knob); 0 keeps the default rule.  Host lists
+// only (touches nothing but W): several class pairs may be listed at once.
+static void list_items(const Plan& p, ClassPairWork& W, int force) {
   const auto& disp = dispatch();
   const int x = W.x, y = W.y;
   const ClassList& X = p.classes[x];
@@ -928,8 +936,6 @@ static void fill_items(Plan& p, ClassPairWork& W, int force) {
     }
   }
   W.nwork = (int)items.size();
-  ++p.layout_gen;
-  upload_items(W.work, W.split, items);
   W.h_items.clear();  // unsharded: the active items are all_items
   W.all_items = std::move(items);
   for (auto* B : W.buckets) delete B;
@@ -972,7 +978,6 @@ static void fill_items(Plan& p, ClassPairWork& W, int force) {
     GenBucket* B = kv.second;
     B->h_items.clear();
     B->nwork = (int)B->all_items.size();
-    upload_items(B->work, B->split, B->all_items);
     const bool bgrp = (B->gb == 1 && B->gk == 1) ? grp
                                                     : (disp.grpg64[cls][gen_slot(B->gb, B->gk)] != nullptr &&
                                                        disp.grpg32[cls][gen_slot(B->gb, B->gk)] != nullptr);
@@ -982,6 +987,58 @@ static void fill_items(Plan& p, ClassPairWork& W, int force) {
     }
     W.buckets.push_back(B);
   }
+}
+
+static void upload_lists(Plan& p, ClassPairWork& W) {
+  ++p.layout_gen;
+  upload_items(W.work, W.split, W.all_items);
+  if (W.use_grp) upload_group(W.grp);
+  for (auto* B : W.buckets) {
+    upload_items(B->work, B->split, B->all_items);
+    if (B->use_grp) upload_group(B->grp);
+  }
+}
+
+static void fill_items(Plan& p, ClassPairWork& W, int force) {
+  list_items(p, W, force);
+  upload_lists(p, W);
+}
+
+// The class pairs of a new plan are listed by up to eight threads, the pairs
+// of the longest lists first: the lists are most of a plan's host time
+// (kPlanPairsPerThread keeps plans of a molecule or two on the caller's
+// thread, where starting threads costs more than it saves).
+constexpr size_t kPlanPairsPerThread = 512;
+static void list_all_items(const Plan& p, std::vector<ClassPairWork*> work) {
+  std::sort(work.begin(), work.end(), [&](const ClassPairWork* a, const ClassPairWork* b) {
+    return p.classes[a->x].pairs.size() * p.classes[a->y].pairs.size() >
+           p.classes[b->x].pairs.size() * p.classes[b->y].pairs.size();
+  });
+  size_t pairs = 0;
+  for (int c = 0; c < kPairClasses; ++c) pairs += p.classes[c].pairs.size();
+  const size_t threads = std::min<size_t>({8, std::max(1u, std::thread::hardware_concurrency()),
+                                           std::max<size_t>(1, pairs / kPlanPairsPerThread), work.size()});
+  dispatch();   // the table is filled before the threads read it
+  std::atomic<size_t> next{0};
+  std::mutex mu;
+  std::exception_ptr failed;
+  auto run = [&] {
+    try {
+      for (size_t i; (i = next++) < work.size();) list_items(p, *work[i], 0);
+    } catch (...) {
+      std::lock_guard<std::mutex> lock(mu);
+      if (!failed) failed = std::current_exception();
+    }
+  };
+  std::vector<std::thread> pool;
+  try {
+    while (pool.size() + 1 < threads) pool.emplace_back(run);
+  } catch (const std::system_error&) {
+    // no more threads to be had: the ones that started and this one do the work
+  }
+  run();
+  for (auto& t : pool) t.join();
+  if (failed) std::rethrow_exception(failed);
 }
 
 // Restrict class pair W to the plan's shard: contiguous cost-balanced blocks
@@ -1524,17 +1581,24 @@ static Plan* build_plan(const b200jk_molecule* mols, int nmol, int cart, double 
     build_bra_order(L);
   }
   // ---- work items per class pair (X >= Y)
+  std::vector<std::unique_ptr<ClassPairWork>> listed;
+  std::vector<ClassPairWork*> todo;
   for (int x = 0; x < kPairClasses; ++x)
     for (int y = 0; y <= x; ++y) {
       if (p.classes[x].pairs.empty() || p.classes[y].pairs.empty()) continue;
-      auto* W = new ClassPairWork();
+      listed.emplace_back(new ClassPairWork());
+      ClassPairWork* W = listed.back().get();
       W->x = x;
       W->y = y;
       W->nbra = (int)p.classes[x].pairs.size();
-      fill_items(p, *W, 0);
-      if (W->nwork == 0) { delete W; continue; }
-      p.work.push_back(W);
+      todo.push_back(W);
     }
+  list_all_items(p, todo);
+  for (auto& W : listed) {
+    if (W->nwork == 0) continue;
+    upload_lists(p, *W);
+    p.work.push_back(W.release());
+  }
   // ---- quartet count on the reference's shells (parent pairs, canonical)
   {
     long long total = 0;
