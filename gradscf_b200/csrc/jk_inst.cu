@@ -29,9 +29,15 @@ struct Policy {
   using CI = ClassInfo<LA, LB, LC, LD>;
   // FP32 blocks take half the registers of FP64 ones: a larger register-path
   // limit (measured on (H2O)32 cc-pVDZ: (11|11), (21|11), (21|20), (22|10)
-  // run 3-6x faster there than on the tile path)
-  static constexpr int LIMIT = sizeof(R) == 4 ? B200JK_REG_LIMIT32 : 96;
-  static constexpr bool REG = (3 * CI::NG + CI::NOUT <= LIMIT) && CI::NROOT <= 3;
+  // run 3-6x faster there than on the tile path).  FP64 blocks above 96 spill,
+  // and up to 165 still beat the tile path, whose lanes read their operands
+  // from shared memory: FP64 class times of (H2O)32 cc-pVDZ (11|11) 4.8 -> 1.7 ms,
+  // (22|10) 2.3 -> 0.9, (21|20) 3.1 -> 2.4; its FP64 build 75.5 -> 70.2 ms.
+  static constexpr int SIZE = 3 * CI::NG + CI::NOUT;
+  static constexpr bool REG = SIZE <= (sizeof(R) == 4 ? B200JK_REG_LIMIT32 : 165) && CI::NROOT <= 3;
+  // bra groups and grouped lists hold several blocks or pass sums per lane:
+  // only where the block itself leaves registers for them
+  static constexpr bool LISTS = REG && SIZE <= (sizeof(R) == 4 ? B200JK_REG_LIMIT32 : 96);
   static constexpr int TEAM = CI::NOUT <= 4 * 24 ? 4 : CI::NOUT <= 8 * 24 ? 8 : CI::NOUT <= 16 * 24 ? 16 : 32;
 };
 
@@ -201,7 +207,7 @@ constexpr int YA = pc_la(Y), YB = pc_lb(Y);
 
 // Grouped lists: both precisions on the register path and an (l, 0) side;
 // up to 4 combinations on a (0, 0) pair, 2 on other (l, 0) pairs.
-constexpr bool GROUPED = Policy<XA, XB, YA, YB, float>::REG && Policy<XA, XB, YA, YB>::REG && (XB == 0 || YB == 0);
+constexpr bool GROUPED = Policy<XA, XB, YA, YB, float>::LISTS && Policy<XA, XB, YA, YB>::LISTS && (XB == 0 || YB == 0);
 
 constexpr int gslot(int g) { return g == 1 ? 0 : (g == 2 ? 1 : 2); }
 
@@ -211,7 +217,7 @@ constexpr int gslot(int g) { return g == 1 ? 0 : (g == 2 ? 1 : 2); }
 #endif
 // The per-lane pass sums (GrpAcc::N values of 32 lanes, 4 warps) stay within
 // 32 KB of static shared memory in FP64.
-constexpr bool GRP = B200JK_GRP && Policy<XA, XB, YA, YB, float>::REG && Policy<XA, XB, YA, YB>::REG &&
+constexpr bool GRP = B200JK_GRP && Policy<XA, XB, YA, YB, float>::LISTS && Policy<XA, XB, YA, YB>::LISTS &&
                      GrpAcc<XA, XB, YA, YB>::N <= 32;
 #ifndef B200JK_GRP_GEN
 #define B200JK_GRP_GEN 1
