@@ -126,13 +126,16 @@ inline int persistent_blocks(Kernel* kernel, int threads, size_t smem, std::atom
   return v;
 }
 
-// Dynamic shared memory above 48 KB is an opt-in attribute of each kernel in
-// each device's context: set it on the current device the first time a
-// kernel is launched there (bit d of `done` marks device d; any thread).
+// A block's shared memory, static and dynamic together, above 48 KB is an
+// opt-in attribute of each kernel in each device's context: set it on the
+// current device the first time a kernel is launched there (bit d of `done`
+// marks device d; any thread).  It is set for every amount of dynamic memory:
+// what a kernel holds statically counts too, so a launch of less than 48 KB
+// can need it (the geometry products of (32|22): 47.7 KB beside 0.8 KB).
 // Returns the attribute call's error (cudaSuccess when nothing was needed).
 template <typename Kernel>
 inline cudaError_t smem_opt_in(Kernel* kernel, size_t bytes, std::atomic<uint64_t>& done) {
-  if (bytes <= 48 * 1024) return cudaSuccess;
+  if (bytes == 0) return cudaSuccess;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
