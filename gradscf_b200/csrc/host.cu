@@ -1626,11 +1626,7 @@ static Plan* build_plan(const b200jk_molecule* mols, int nmol, int cart, double 
     p.quartets = total;
   }
   CUDA_OK(p.d_queue.ensure(kQueueSlots * sizeof(int)));
-  for (int i = 0; i < kAuxStreams; ++i) {
-    CUDA_OK(cudaStreamCreateWithFlags(&p.aux[i], cudaStreamNonBlocking));
-    CUDA_OK(cudaEventCreateWithFlags(&p.join_ev[i], cudaEventDisableTiming));
-  }
-  CUDA_OK(cudaEventCreateWithFlags(&p.fork_ev, cudaEventDisableTiming));
+  p.aux.create();
   return plan.release();
 }
 
@@ -1783,34 +1779,24 @@ static long long jk_cost(const ClassPairWork& W) {
 }
 
 // Independent class-pair launches spread over the caller's stream and the
-// plan's auxiliary streams (forked from and joined back into `st`):
-// longest-first onto the least-loaded stream; `serial` keeps them on `st`.
+// plan's auxiliary streams, longest-first onto the least-loaded stream;
+// `serial` keeps them on `st`.
 template <typename F>
 static void spread_classes(Plan& p, cudaStream_t st, bool serial, F&& launch) {
-  const int nstreams = serial ? 1 : kAuxStreams + 1;
-  cudaStream_t streams[kAuxStreams + 1] = {st};
-  for (int i = 0; i < kAuxStreams; ++i) streams[i + 1] = p.aux[i];
-  if (!serial) {
-    CUDA_OK(cudaEventRecord(p.fork_ev, st));
-    for (int i = 0; i < kAuxStreams; ++i) CUDA_OK(cudaStreamWaitEvent(p.aux[i], p.fork_ev, 0));
-  }
   std::vector<std::pair<long long, ClassPairWork*>> order;
   for (auto* W : p.work)
     if (W->nwork > 0) order.push_back({W->prim_quartets, W});
   std::sort(order.begin(), order.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
-  std::vector<long long> load(nstreams, 0);
+  StreamFork streams(serial ? nullptr : &p.aux, st);
+  std::vector<long long> load(streams.count(), 0);
   for (auto& [cost, W] : order) {
     int best = 0;
-    for (int i = 1; i < nstreams; ++i)
+    for (int i = 1; i < streams.count(); ++i)
       if (load[i] < load[best]) best = i;
     load[best] += cost;
     launch(*W, streams[best]);
   }
-  if (!serial)
-    for (int i = 0; i < kAuxStreams; ++i) {
-      CUDA_OK(cudaEventRecord(p.join_ev[i], p.aux[i]));
-      CUDA_OK(cudaStreamWaitEvent(st, p.join_ev[i], 0));
-    }
+  streams.join();
 }
 
 // The class-pair launches of one build spread over the caller's stream and
@@ -1819,14 +1805,11 @@ static void spread_classes(Plan& p, cudaStream_t st, bool serial, F&& launch) {
 // low-occupancy kernels overlap.  Longest-first onto the least-loaded
 // stream; in split builds the FP64 slices share one auxiliary stream.
 static void launch_all(Plan& p, JKArgs a, int precision, cudaStream_t st) {
-  CUDA_OK(cudaEventRecord(p.fork_ev, st));
-  for (int i = 0; i < kAuxStreams; ++i) CUDA_OK(cudaStreamWaitEvent(p.aux[i], p.fork_ev, 0));
-  cudaStream_t streams[kAuxStreams + 1] = {st};
-  for (int i = 0; i < kAuxStreams; ++i) streams[i + 1] = p.aux[i];
   std::vector<std::pair<long long, ClassPairWork*>> order;
   for (auto* W : p.work) order.push_back({jk_cost(*W), W});
   std::sort(order.begin(), order.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
   const bool split = precision == B200JK_SPLIT;  // split builds: stream 1 carries the FP64 slices
+  StreamFork streams(&p.aux, st);
   std::vector<long long> load(kAuxStreams + 1, 0);
   for (auto& [cost, W] : order) {
     int best = -1;
@@ -1838,10 +1821,7 @@ static void launch_all(Plan& p, JKArgs a, int precision, cudaStream_t st) {
     launch_units(p, *W, a, precision, streams[best], false, split ? 2 : -1);
     if (split) launch_units(p, *W, a, precision, streams[1], false, 1);
   }
-  for (int i = 0; i < kAuxStreams; ++i) {
-    CUDA_OK(cudaEventRecord(p.join_ev[i], p.aux[i]));
-    CUDA_OK(cudaStreamWaitEvent(st, p.join_ev[i], 0));
-  }
+  streams.join();
 }
 
 // The J/K pipeline on caller-provided scratch: dens/dens_f hold (hermi ? nb :

@@ -8,6 +8,7 @@
 
 #include "common.cuh"
 #include "dispatch.h"
+#include "streams.h"
 
 namespace b200jk {
 
@@ -120,16 +121,11 @@ struct ProfileEvent {
   cudaEvent_t start, stop;
 };
 
-#ifndef B200JK_AUX_STREAMS
-#define B200JK_AUX_STREAMS 3
-#endif
-constexpr int kAuxStreams = B200JK_AUX_STREAMS;  // streams besides the caller's for concurrent class-pair launches
 constexpr int kQueueSlots = 4096;  // work-queue counters of persistent launches, reused cyclically
 
 struct Plan {
   int device = 0;
-  cudaStream_t aux[kAuxStreams] = {};
-  cudaEvent_t fork_ev = nullptr, join_ev[kAuxStreams] = {};
+  AuxStreams aux;
   int shard_rank = 0, shard_world = 1;  // active work-item shard
   int cart = 0;
   double cutoff = 0.0;
@@ -186,11 +182,6 @@ struct Plan {
   bool profiling = false;
   std::vector<ProfileEvent> events;
   ~Plan() {
-    for (int i = 0; i < kAuxStreams; ++i) {
-      if (aux[i]) cudaStreamDestroy(aux[i]);
-      if (join_ev[i]) cudaEventDestroy(join_ev[i]);
-    }
-    if (fork_ev) cudaEventDestroy(fork_ev);
     for (auto* w : work) delete w;
     for (auto& e : events) {
       cudaEventDestroy(e.start);
