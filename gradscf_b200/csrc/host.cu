@@ -12,6 +12,7 @@
 #include <memory>
 #include <mutex>
 #include <numeric>
+#include <optional>
 #include <stdexcept>
 #include <string>
 #include <system_error>
@@ -1779,15 +1780,15 @@ static long long jk_cost(const ClassPairWork& W) {
 }
 
 // Independent class-pair launches spread over the caller's stream and the
-// plan's auxiliary streams, longest-first onto the least-loaded stream;
-// `serial` keeps them on `st`.
+// streams of `aux` (null: `st` alone), longest-first onto the least-loaded
+// stream.
 template <typename F>
-static void spread_classes(Plan& p, cudaStream_t st, bool serial, F&& launch) {
+static void spread_classes(const Plan& p, AuxStreams* aux, cudaStream_t st, F&& launch) {
   std::vector<std::pair<long long, ClassPairWork*>> order;
   for (auto* W : p.work)
     if (W->nwork > 0) order.push_back({W->prim_quartets, W});
   std::sort(order.begin(), order.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
-  StreamFork streams(serial ? nullptr : &p.aux, st);
+  StreamFork streams(aux, st);
   std::vector<long long> load(streams.count(), 0);
   for (auto& [cost, W] : order) {
     int best = 0;
@@ -2422,7 +2423,14 @@ int b200jk_packed_eri(b200jk_plan* plan, int32_t layout, double* d_out, int64_t 
     CUDA_OK(cudaMemsetAsync(d_out, 0, (size_t)size * sizeof(double), st));
     JKArgs a = base_args(p);
     const auto& disp = dispatch();
-    spread_classes(p, st, false, [&](ClassPairWork& W, cudaStream_t ls) {
+    // the call reads the plan alone, so calls on one plan may overlap from any
+    // threads and streams: the launches spread over streams of their own, and
+    // stay on the caller's while it is captured
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    CUDA_OK(cudaStreamIsCapturing(st, &capture));
+    std::optional<StreamPool::Lease> lease;
+    if (capture == cudaStreamCaptureStatusNone) lease.emplace(p.eri_streams);
+    spread_classes(p, lease ? lease->get() : nullptr, st, [&](ClassPairWork& W, cudaStream_t ls) {
       set_lists(a, p, W);
       a.work = W.work.as<int4>();
       a.nwork = W.nwork;
@@ -2509,7 +2517,7 @@ int b200jk_direct_jk_geom_vjp_precision(b200jk_plan* plan, const double* d_densi
     a.grad = d_grad;
     const auto& disp = dispatch();
     // serial while profiling, so each launch is timed alone
-    spread_classes(p, st, p.profiling, [&](ClassPairWork& W, cudaStream_t ls) {
+    spread_classes(p, p.profiling ? nullptr : &p.aux, st, [&](ClassPairWork& W, cudaStream_t ls) {
       const int cls = quartet_class(W.x, W.y);
       set_lists(a, p, W);
       a.work = W.work.as<int4>();
@@ -2542,7 +2550,7 @@ int b200jk_direct_jk_geom_vjp_precision(b200jk_plan* plan, const double* d_densi
 // of every class pair's expanded work items, on `a` as prepared by the caller.
 static void launch_geom_all(Plan& p, JKArgs a, int mode, cudaStream_t st) {
   a.split_mode = 0;
-  spread_classes(p, st, false, [&](ClassPairWork& W, cudaStream_t ls) {
+  spread_classes(p, &p.aux, st, [&](ClassPairWork& W, cudaStream_t ls) {
     set_lists(a, p, W);
     a.work = W.work.as<int4>();
     a.nwork = W.nwork;

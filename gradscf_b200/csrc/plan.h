@@ -125,7 +125,8 @@ constexpr int kQueueSlots = 4096;  // work-queue counters of persistent launches
 
 struct Plan {
   int device = 0;
-  AuxStreams aux;
+  AuxStreams aux;          // of calls that use the plan's scratch, which callers order
+  StreamPool eri_streams;  // of packed ERI calls, which only read the plan
   int shard_rank = 0, shard_world = 1;  // active work-item shard
   int cart = 0;
   double cutoff = 0.0;

@@ -3,8 +3,13 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <cstddef>
+#include <memory>
+#include <mutex>
 #include <stdexcept>
 #include <string>
+#include <utility>
+#include <vector>
 
 namespace b200jk {
 
@@ -38,6 +43,51 @@ struct AuxStreams {
     }
     if (fork) cudaEventDestroy(fork);
   }
+};
+
+// Sets for calls that share nothing else and may overlap from any threads and
+// streams: each holds a set of its own (two records of one fork event between
+// a record and its waits would drop the order of the first).  Up to kKeep
+// idle sets stay for the next call, whose work then queues behind what is
+// still running on them.
+class StreamPool {
+ public:
+  class Lease {
+   public:
+    explicit Lease(StreamPool& pool) : pool_(pool), set_(pool.take()) {}
+    ~Lease() { pool_.give_back(std::move(set_)); }
+    Lease(const Lease&) = delete;
+    Lease& operator=(const Lease&) = delete;
+    AuxStreams* get() const { return set_.get(); }
+
+   private:
+    StreamPool& pool_;
+    std::unique_ptr<AuxStreams> set_;
+  };
+  StreamPool() { idle_.reserve(kKeep); }
+
+ private:
+  static constexpr size_t kKeep = 4;
+  std::unique_ptr<AuxStreams> take() {
+    std::unique_ptr<AuxStreams> set;
+    {
+      std::lock_guard<std::mutex> lock(mu_);
+      if (!idle_.empty()) {
+        set = std::move(idle_.back());
+        idle_.pop_back();
+        return set;
+      }
+    }
+    set.reset(new AuxStreams());
+    set->create();
+    return set;
+  }
+  void give_back(std::unique_ptr<AuxStreams> set) {
+    std::lock_guard<std::mutex> lock(mu_);
+    if (idle_.size() < kKeep) idle_.push_back(std::move(set));   // else destroyed; its work still completes
+  }
+  std::mutex mu_;
+  std::vector<std::unique_ptr<AuxStreams>> idle_;
 };
 
 // The streams of `aux` forked from `st` for the life of this object.  join()

@@ -120,7 +120,8 @@ int b200jk_plan_profile(b200jk_plan* plan, double* ms64, double* ms32, int32_t* 
  * np = n(n+1)/2 output AO pairs, pair(i,j) = i(i+1)/2 + j for i >= j.
  * out_size must equal the layout's element count.  d_out is zeroed first;
  * quartets below the plan's Schwarz cut stay zero (the reference uses
- * cut 0 here). */
+ * cut 0 here).  The call only reads the plan and works on streams of its own
+ * that it joins into `stream`, so calls on one plan may overlap. */
 int b200jk_packed_eri(b200jk_plan* plan, int32_t layout, double* d_out, int64_t out_size, void* stream);
 
 /* J/K from packed ERIs (replaces PackedJK, csrc/packed_jk.cc:6-80): d_eri in

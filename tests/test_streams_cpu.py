@@ -1,5 +1,5 @@
 """Forked launch streams (csrc/streams.h) against a recording stand-in for the CUDA runtime: whatever leaves the
-scope, the caller's stream waits for every stream that was forked."""
+scope, the caller's stream waits for every stream that was forked; calls that overlap hold different sets."""
 import os
 import subprocess
 from pathlib import Path
@@ -86,6 +86,48 @@ int main() {
 }
 """
 
+POOL = r"""
+#include "streams.h"
+#include <cstdio>
+#include <thread>
+using namespace b200jk;
+
+int main() {
+  int bad = 0;
+  {
+    StreamPool pool;
+    AuxStreams *a, *b;
+    {
+      StreamPool::Lease x(pool), y(pool);   // two calls at a time
+      a = x.get();
+      b = y.get();
+      if (a == b || a->fork == b->fork || a->s[0] == b->s[0]) ++bad;
+    }
+    StreamPool::Lease z(pool);              // a later call takes an idle set
+    if (z.get() != a && z.get() != b) ++bad;
+    // interleaved as two threads may be: B's fork is recorded between A's record and A's waits
+    FakeStream sa, sb;
+    const int work = queue_op(&sa);
+    StreamPool::Lease w(pool);
+    cudaEventRecord(z.get()->fork, &sa);
+    cudaEventRecord(w.get()->fork, &sb);
+    cudaStreamWaitEvent(z.get()->s[0], z.get()->fork, 0);
+    if (!z.get()->s[0]->done.count(work)) ++bad;
+  }
+  if (g_live != 0) ++bad;
+  {
+    StreamPool pool;                        // idle sets are bounded
+    std::vector<std::unique_ptr<StreamPool::Lease>> held;
+    for (int i = 0; i < 9; ++i) held.emplace_back(new StreamPool::Lease(pool));
+    held.clear();
+    if (g_live != 4 * (2 * kAuxStreams + 1)) ++bad;
+  }
+  if (g_live != 0) ++bad;
+  if (bad) std::printf("%d failed\n", bad);
+  return bad;
+}
+"""
+
 
 @pytest.fixture(scope="module")
 def runtime(tmp_path_factory):
@@ -105,3 +147,7 @@ def run(root, source, name):
 
 def test_every_exit_of_a_fork_joins_its_streams(runtime):
     run(runtime, MAIN, "fork")
+
+
+def test_overlapping_calls_hold_different_streams(runtime):
+    run(runtime, POOL, "pool")
