@@ -1,9 +1,7 @@
 // Plan construction, basis transforms, J/K orchestration and the C ABI.
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstring>
-#include <exception>
 #include <map>
 #include <unordered_map>
 #include <set>
@@ -15,12 +13,12 @@
 #include <optional>
 #include <stdexcept>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <tuple>
 #include <vector>
 
 #include "../../include/b200jk.h"
+#include "host_threads.h"
 #include "jk_kernels.cuh"
 #include "plan.h"
 #include "rys_tables.h"
@@ -1020,26 +1018,7 @@ static void list_all_items(const Plan& p, std::vector<ClassPairWork*> work) {
   const size_t threads = std::min<size_t>({8, std::max(1u, std::thread::hardware_concurrency()),
                                            std::max<size_t>(1, pairs / kPlanPairsPerThread), work.size()});
   dispatch();   // the table is filled before the threads read it
-  std::atomic<size_t> next{0};
-  std::mutex mu;
-  std::exception_ptr failed;
-  auto run = [&] {
-    try {
-      for (size_t i; (i = next++) < work.size();) list_items(p, *work[i], 0);
-    } catch (...) {
-      std::lock_guard<std::mutex> lock(mu);
-      if (!failed) failed = std::current_exception();
-    }
-  };
-  std::vector<std::thread> pool;
-  try {
-    while (pool.size() + 1 < threads) pool.emplace_back(run);
-  } catch (const std::system_error&) {
-    // no more threads to be had: the ones that started and this one do the work
-  }
-  run();
-  for (auto& t : pool) t.join();
-  if (failed) std::rethrow_exception(failed);
+  run_indexed(work.size(), threads, [&](size_t i) { list_items(p, *work[i], 0); });
 }
 
 // Restrict class pair W to the plan's shard: contiguous cost-balanced blocks
