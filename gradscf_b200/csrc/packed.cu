@@ -316,8 +316,7 @@ void check_packed(const double* d_eri, int layout, int64_t eri_size, int n, cons
   const long long np = (long long)n * (n + 1) / 2;
   if (eri_size != (layout == 1 ? np * (np + 1) / 2 : np * np))
     fail_invalid("Packed J/K dimensions do not match");  // csrc/packed_jk.cc:18-22
-  if (with_k && (size_t)4 * n * nb * sizeof(double) > kMaxShared)
-    fail_invalid("Packed J/K: n x nb too large for the per-row exchange sums (n * nb <= 6400)");
+  // a warp's exchange sums of one density (the passes take densities one or two at a time)
   if (with_k && packed_k_warp(n, 1) * sizeof(double) > kMaxShared)
     fail_invalid("Packed J/K: n too large for one row's exchange sums");
 }

@@ -1,5 +1,5 @@
 """Packed J/K at the edges of its tiles (32 x 32 of a row's triangle, 1024 columns and 128 rows of the pair
-matrix) and of its density groups (three for J, two for K), s4 and s8, symmetric and nonsymmetric densities,
+matrix) and of its density groups (three for J, two for K; no limit on their number), s4 and s8, symmetric and nonsymmetric densities,
 against torch on the unpacked integrals.  The integrals need no basis: any symmetric pair matrix.  Both sides
 sum up to n^2 products of order one in FP64; 4 n^2 eps max|element| bounds their difference."""
 import sys
@@ -17,7 +17,8 @@ from gradscf_b200 import jk as J  # noqa: E402
 
 @pytest.mark.parametrize("layout", ["s4", "s8"])
 @pytest.mark.parametrize("hermi", [True, False])
-@pytest.mark.parametrize("n,nb", [(1, 1), (2, 3), (7, 2), (31, 1), (32, 4), (33, 2), (45, 5), (64, 1), (65, 3)])
+@pytest.mark.parametrize("n,nb", [(1, 1), (2, 3), (7, 2), (31, 1), (32, 4), (33, 2), (45, 5), (64, 1), (65, 3),
+                                  (33, 200)])   # a batch of more than 6400 rows
 def test_packed_jk_shapes(n, nb, hermi, layout):
     gen = torch.Generator(device="cuda").manual_seed(n * 8 + nb)
     npair = n * (n + 1) // 2
