@@ -18,9 +18,10 @@ from gradscf_b200 import jk as J  # noqa: E402
 from tests.gpu_util import psd_density, tables  # noqa: E402
 
 
-@pytest.mark.parametrize("cart", [False, True])
-def test_geometry_products_of_every_class_match_differences(cart):
+@pytest.mark.parametrize("cart,omega", [(False, 0.0), (True, 0.0), (False, 0.33)])
+def test_geometry_products_of_every_class_match_differences(cart, omega):
     top, par, sa, atm, bas, env = tables("O 0 0 0; H 0.1 0.7572 0.5865", "cc-pvtz", cart)
+    env[8] = omega
     rng = np.random.default_rng(3)
     d = psd_density(top.nao, 5, 2)
     slots = (atm[:, 1][:, None] + np.arange(3)[None, :]).ravel()

@@ -1,7 +1,7 @@
 """The tile path (blocks that do not fit one thread's registers: d and f shells): J, K and their combinations against
 the packed integrals, contracted in torch.  Both sum the same n^2 FP64 products per element, in another order:
 n^2 eps |element| < 1e-11 here.  Two waters give items whose last pass is ragged for every number of quartets a
-block takes (1 to 14), triple zeta every class up to (ff|ff)."""
+block takes (12, 7, 4, 3, 2 or 1), triple zeta every class up to (ff|ff).  Split-precision bounds: test_small_builds_gpu."""
 import sys
 from pathlib import Path
 
@@ -16,7 +16,7 @@ sys.path.insert(0, str(Path(__file__).resolve().parents[1]))
 from gradscf_b200 import jk as J  # noqa: E402
 from gradscf_b200 import workloads as W  # noqa: E402
 from tests.gpu_util import tables  # noqa: E402
-from tests.test_small_builds_gpu import packed_to_full  # noqa: E402
+from tests.test_small_builds_gpu import PRECISIONS, packed_to_full  # noqa: E402
 
 
 @pytest.fixture(scope="module", params=[(2, "cc-pvtz", False), (1, "cc-pvtz", True), (2, "cc-pvdz", True)])
@@ -30,15 +30,15 @@ def molecule(request):
 @pytest.mark.parametrize("with_j,with_k,hermi,nb", [(True, True, True, 1), (True, False, True, 3),
                                                     (False, True, True, 2), (True, True, False, 3),
                                                     (False, True, False, 1)])
-@pytest.mark.parametrize("precision,tol", [("fp64", 1e-11), ("split", 2e-6)])   # split: FP32 quartets below 1e-6
-def test_tile_classes_match_packed_integrals(molecule, with_j, with_k, hermi, nb, precision, tol):
+@pytest.mark.parametrize("precision,cut,tol,rel", PRECISIONS)
+def test_tile_classes_match_packed_integrals(molecule, with_j, with_k, hermi, nb, precision, cut, tol, rel):
     mol, cart, n, eri = molecule
     rng = np.random.default_rng(nb)
     d = torch.as_tensor(rng.normal(size=(nb, n, n)) / n, device=eri.device)
     if hermi:
         d = d + d.transpose(1, 2)
-    j, k = J.DirectJKPlan([mol], cart=cart).jk(d, with_j=with_j, with_k=with_k, hermi=hermi, precision=precision)
-    if with_j:
-        assert (j - torch.einsum("pqrs,ers->epq", eri, d)).abs().max().item() < tol
-    if with_k:
-        assert (k - torch.einsum("prqs,ers->epq", eri, d)).abs().max().item() < tol
+    j, k = J.DirectJKPlan([mol], cart=cart).jk(d, with_j=with_j, with_k=with_k, hermi=hermi, precision=precision,
+                                               fp32_cut=cut)
+    for on, x, path in ((with_j, j, "pqrs,ers->epq"), (with_k, k, "prqs,ers->epq")):
+        y = torch.einsum(path, eri, d)
+        assert not on or (x - y).abs().max().item() < tol + rel * y.abs().max().item()
