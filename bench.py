@@ -27,6 +27,8 @@ as many as fit in about 150 s, at least one, after a warm-up build of the
 water monomer).  The reference screens by Schwarz bounds only, so its build
 time does not depend on the density's values.  The `cpu_baseline` object of
 the GPU line is a bounded sample instead: one build of the first 8 waters.
+Where oracle/_ref was not built (it needs the reference's sources) both say
+that they are unavailable, and the GPU arm's own numbers stand.
 
 Multi-GPU (torchrun): one J/K build is shared by the ranks (strong scaling):
 each rank evaluates its cost-balanced block of every class pair's work items
@@ -52,6 +54,14 @@ METRIC = "J/K build s/iter & ERI quartets/s: split vs FP64 on B200 at |ΔE|≤1e
 WORKLOAD = "(H2O)32 cc-pVDZ direct J/K (768 sph AOs), Schwarz 1e-12, seed 1"
 FP32_CUT = 1e-6
 SAMPLE_WATERS = 8
+
+
+def reference_unavailable():
+    """Why the CPU reference cannot run here (one line), or None."""
+    import oracle
+    if oracle.LIB_PATH.is_file():
+        return None
+    return "oracle/_ref is not built: the reference's sources (vendored libcint) are not on this machine"
 
 
 def sample_workload():
@@ -189,6 +199,10 @@ def main():
 
     if args.impl == "reference":
         if rank != 0:
+            return 0
+        why = reference_unavailable()
+        if why:
+            print(json.dumps({"impl": "reference", "unavailable": why}))
             return 0
         value, cores, sample, step_s, nbuilds = cpu_reference_full(args.steps)
         line = {"metric": METRIC, "value": value, "unit": "quartets/s", "n_gpus": args.gpus,
@@ -413,9 +427,13 @@ def main():
             return out
         line["class_ms_per_step"] = {"split": _ct("split"), "fp64": _ct("fp64")}
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
-        value, cores, sample, _ = cpu_reference_run(1, 0)
-        line["cpu_baseline"] = {"value": value, "unit": "quartets/s", "cores": cores,
-                                "kind": "reference", "sample": sample}
+        why = reference_unavailable()
+        if why:
+            line["cpu_baseline"] = {"unavailable": why}
+        else:
+            value, cores, sample, _ = cpu_reference_run(1, 0)
+            line["cpu_baseline"] = {"value": value, "unit": "quartets/s", "cores": cores,
+                                    "kind": "reference", "sample": sample}
     if rank == 0:
         print(json.dumps(line))
     plan.close()
