@@ -294,8 +294,10 @@ __device__ __forceinline__ void raised_bra(R ab, const R* w, int q, R* G) {
 // (value, d/dA, d/dB, d/dC) per (unit, axis, unraised index tuple) -- four
 // values side by side, one or two 16-byte loads -- and sums the nine centre
 // partials over the (unit, element) pairs; Gamma stays in shared memory per
-// quartet.  What bounds these classes is latency (few quartets, long chains):
-// the forms this replaces built one primitive quartet's tables on 3 N threads
+// quartet.  What bounds it is shared memory: three quads (96 bytes in FP64) feed
+// fifteen operations of a (unit, element) pair.  Under ncu, (H2O)4 cc-pVTZ FP64
+// (22|10) has the L1 data stage 82% busy (44% of the shared wavefronts are bank
+// conflicts) beside 15% of the FP64 pipe.  The forms this replaces built one primitive quartet's tables on 3 N threads
 // at a time and recomputed each element's derivative factors from the table.
 // (H2O)4 cc-pVTZ split VJP 42.2 -> 33.9 ms (serial class times 70 -> 40).
 // ---------------------------------------------------------------------------
@@ -489,9 +491,13 @@ struct GradLane {
 #ifndef B200JK_GRAD_LANE_TABLES
 #define B200JK_GRAD_LANE_TABLES 90   // doubles of one centre's three tables
 #endif
-  // measured on (H2O)16 cc-pVTZ: 1.5-2.6x over the team kernel up to 90
-  // elements, slower than the register kernel on its classes and than the
-  // team kernel on 108-element blocks
+  // (H2O)8 cc-pVTZ FP64 class times, this kernel against grad_unit_kernel: all
+  // eleven classes inside the line are faster here, from (11|11) 3.0 against
+  // 5.2 ms and (20|11) 6.3 / 21.2 to (31|00) 1.6 / 6.7 (the whole VJP 269 / 348 ms,
+  // split 236 / 281).  With the line at 110 elements and 162 doubles (30|11)
+  // 4.5 -> 3.1 ms and (22|10) 11.4 -> 10.5, but (30|30) 1.13 -> 1.30, the whole VJP
+  // unchanged and the split one 236 -> 242 ms: the line stays.  Classes that fit
+  // the register kernel were slower here (0.83-0.87x, (H2O)16 cc-pVTZ).
   static constexpr bool OK = !GradReg<LA, LB, LC, LD>::OK && CI::NOUT <= 90 && 3 * NGMAX <= B200JK_GRAD_LANE_TABLES;
 };
 

@@ -2158,7 +2158,7 @@ int b200jk_plan_autotune(b200jk_plan* plan, const double* d_density, int32_t nb,
     if (chunks) std::fill(chunks, chunks + kQuartetClasses, -1);
     for (auto* W : p.work) {
       const int cls = quartet_class(W->x, W->y);
-      if (!disp.reg_path[cls]) continue;  // tile / team items keep their sizes
+      if (!disp.reg_path[cls]) continue;  // tile items keep their sizes
       int best = 0;
       float best_ms = 0.f;
       for (const int cand : {32, 64, 128}) {

@@ -186,7 +186,8 @@ int launch_grad(const JKArgs& args, cudaStream_t stream) {
 
 // The geometry products of one class pair: a block per (item, ket stride);
 // items split over gridDim.y blocks until the launch holds about four blocks
-// per resident one (148 x 3 at 64 KB).
+// per resident one (148 x 3 at 64 KB, which all classes but (33|32) and (33|33)
+// keep to).
 template <int LA, int LB, int LC, int LD>
 int launch_geom(const JKArgs& args, int mode, cudaStream_t stream) {
   if (args.nwork <= 0) return 0;

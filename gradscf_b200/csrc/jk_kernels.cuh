@@ -331,8 +331,10 @@ __device__ __forceinline__ long long dm_index(const JKArgs& args, int mol, int a
 // shuffles before digestion, which the group's first lane does.  What bounds
 // a small build is the longest chain of dependent primitive quartets, not
 // throughput: water cc-pVDZ spent 1.5 of its 3.1 ms in one lane walking the
-// 4096 primitive quartets of the oxygen core (ss|ss) block.  T is kept where
-// every lane of the group gets at least two primitive quartets.
+// 4096 primitive quartets of the oxygen core (ss|ss) block.  T doubles while
+// the group's lanes keep at least two primitive quartets each on average (an
+// uneven product gives some one more and some one less: 3 x 3 over T = 4 is
+// 4, 2, 2 and 1).
 // ---------------------------------------------------------------------------
 struct LaneSplit {
   int t = 1, sub = 0;              // lanes per quartet, this lane's index among them
@@ -1885,8 +1887,11 @@ struct TeamSmem {
 // NCD products with D[a][b] per lane, summed over the team's lanes; J[a][b]
 // stays in a register over the item.
 //
-// What bounds it is shared-memory wavefronts: 3 KSTR reads feed 2 NCD
-// operations per root and lane.  The form it replaces built one primitive
+// What bounds it is shared memory: 3 KSTR reads feed 2 NCD operations per root
+// and lane.  Under ncu, (H2O)6 cc-pVTZ FP64 (32|10), (21|21) and (22|21) have the
+// L1 data stage 61 to 70% busy (a fifth to a quarter of the shared wavefronts
+// are bank conflicts) beside 17 to 21% of the FP64 pipe, at 3 warps a scheduler
+// that wait on barriers, fixed latencies and shared loads.  The form it replaces built one primitive
 // quartet's tables on 3 N threads at a time and digested from a staged block
 // (six reads of every element, rows NCD apart on four banks): (H2O)11 cc-pVTZ
 // FP64 class times (21|20) 8.2 -> 5.5 ms, (22|10) 6.8 -> 3.8, (32|10) 4.8 -> 2.8,

@@ -8,7 +8,11 @@
 // and four for K per symmetric density.  The previous form read it once but
 // added J[c][d] to memory per element and reduced K[a][c] over a warp for
 // every c: 5.82 ms for n = 168, two densities (807 MB).  Here J and K are two
-// passes, each bound by the read: 0.77 ms at that size.
+// passes that read it once each: 0.77 ms at that size, three times what the two
+// reads take at the copy rate.  Under ncu the J pass (0.27 ms) reads 3.0 TB/s and
+// the K pass (0.50 ms) 1.6 TB/s: two warps a scheduler (176 and 168 registers)
+// wait on fixed latencies and on their loads, in K with the L1 data stage 54%
+// busy from the tiles' transposes and broadcast reads.
 //   J: J = M x with M the symmetric pair matrix, x_cd = D_cd + D_dc.  A block
 //      takes 128 rows x 1024 columns; a thread keeps its four columns' x and
 //      column sums in registers (one add per column and block), and the row
