@@ -27,8 +27,8 @@
 // (unit, axis, unraised index tuple), then they take the (unit, element)
 // pairs.  The batch fills about 64 KB of shared memory (three blocks an SM); where
 // one unit beside the accumulators is more, a block takes that: (32|32) and
-// (33|22) 69 KB, (33|32) 100 (two blocks), (33|33) 150 (one).  Under ncu the (00|00) and (10|00) launches of
-// (H2O)2 6-31G* have 2 to 3 warps a scheduler, waiting on the batch's barriers
+// (33|22) 69 KB, (33|32) 100 (two blocks), (33|33) 150 (one).  Under ncu the
+// (00|00) and (10|00) launches of (H2O)2 6-31G* have 2 to 3 warps a scheduler, waiting on the batch's barriers
 // and on fixed latencies, the FP64 pipe 20 to 23% busy.
 // (H2O)2 6-31G* Hessian-vector product: 120.9 -> 1.55 ms.
 #pragma once

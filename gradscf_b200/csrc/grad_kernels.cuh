@@ -297,8 +297,9 @@ __device__ __forceinline__ void raised_bra(R ab, const R* w, int q, R* G) {
 // quartet.  What bounds it is shared memory: three quads (96 bytes in FP64) feed
 // fifteen operations of a (unit, element) pair.  Under ncu, (H2O)4 cc-pVTZ FP64
 // (22|10) has the L1 data stage 82% busy (44% of the shared wavefronts are bank
-// conflicts) beside 15% of the FP64 pipe.  The forms this replaces built one primitive quartet's tables on 3 N threads
-// at a time and recomputed each element's derivative factors from the table.
+// conflicts) beside 15% of the FP64 pipe.  The forms this replaces built one
+// primitive quartet's tables on 3 N threads at a time and recomputed each
+// element's derivative factors from the table.
 // (H2O)4 cc-pVTZ split VJP 42.2 -> 33.9 ms (serial class times 70 -> 40).
 // ---------------------------------------------------------------------------
 template <int LA, int LB, int LC, int LD, typename R>

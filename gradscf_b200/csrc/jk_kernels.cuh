@@ -1891,9 +1891,9 @@ struct TeamSmem {
 // and lane.  Under ncu, (H2O)6 cc-pVTZ FP64 (32|10), (21|21) and (22|21) have the
 // L1 data stage 61 to 70% busy (a fifth to a quarter of the shared wavefronts
 // are bank conflicts) beside 17 to 21% of the FP64 pipe, at 3 warps a scheduler
-// that wait on barriers, fixed latencies and shared loads.  The form it replaces built one primitive
-// quartet's tables on 3 N threads at a time and digested from a staged block
-// (six reads of every element, rows NCD apart on four banks): (H2O)11 cc-pVTZ
+// that wait on barriers, fixed latencies and shared loads.  The form it
+// replaces built one primitive quartet's tables on 3 N threads at a time and
+// digested from a staged block (six reads of every element, rows NCD apart on four banks): (H2O)11 cc-pVTZ
 // FP64 class times (21|20) 8.2 -> 5.5 ms, (22|10) 6.8 -> 3.8, (32|10) 4.8 -> 2.8,
 // its split build 83.4 -> 57.3 ms; (H2O)6 cc-pVTZ FP64 25.6 -> 20.2 ms.
 // ---------------------------------------------------------------------------
